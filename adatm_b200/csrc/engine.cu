@@ -113,15 +113,24 @@ Engine::Engine(std::shared_ptr<const DevCoo> coo, std::vector<std::shared_ptr<De
       ADATM_CUDA(cudaMemsetAsync(memo_[g][deg].get(), 0, n * sizeof(float), stream_));
     }
   }
-  uint64_t maxdim = 1;
+  // all factors in one allocation (and their BF16 copies in another), mode
+  // after mode: the contraction walks number their rows from one base
+  uint64_t maxdim = 1, rows = 0;
   for (int m = 0; m < N; ++m) {
     maxdim = std::max(maxdim, coo_->dims[m]);
-    A_[m].alloc((size_t)coo_->dims[m] * ldr_);
-    ADATM_CUDA(cudaMemsetAsync(A_[m].get(), 0, A_[m].bytes(), stream_));
-    if (opt_.factor_type == FactorType::BF16) {
-      Ab_[m].alloc((size_t)coo_->dims[m] * ldr_);
-      ADATM_CUDA(cudaMemsetAsync(Ab_[m].get(), 0, Ab_[m].bytes(), stream_));
-    }
+    rows += coo_->dims[m];
+  }
+  factors_.alloc((size_t)rows * ldr_);
+  ADATM_CUDA(cudaMemsetAsync(factors_.get(), 0, factors_.bytes(), stream_));
+  if (opt_.factor_type == FactorType::BF16) {
+    factors16_.alloc((size_t)rows * ldr_);
+    ADATM_CUDA(cudaMemsetAsync(factors16_.get(), 0, factors16_.bytes(), stream_));
+  }
+  rows = 0;
+  for (int m = 0; m < N; ++m) {
+    A_[m] = factors_.get() + (size_t)rows * ldr_;
+    Ab_[m] = factors16_.get() ? factors16_.get() + (size_t)rows * ldr_ : nullptr;
+    rows += coo_->dims[m];
     G_[m].alloc((size_t)R_ * R_);
   }
   M_.alloc((size_t)maxdim * ldr_);
@@ -474,7 +483,7 @@ LevelFactors Engine::level_factors(int g, FactorType ft) const {
   const DevCsf &c = *csf_[g];
   for (int l = 0; l < c.nmodes; ++l) {
     const int m = (int)c.dim_perm[l];
-    f.U[l] = ft == FactorType::BF16 ? (const void *)Ab_[m].get() : (const void *)A_[m].get();
+    f.U[l] = ft == FactorType::BF16 ? (const void *)Ab_[m] : (const void *)A_[m];
   }
   return f;
 }
@@ -522,7 +531,7 @@ double Engine::mttkrp_bytes(int mode) const {
 
 void Engine::init_factors(uint64_t seed) {
   for (int m = 0; m < coo_->nmodes; ++m)
-    factor_init_device(A_[m].get(), Ab_[m].get(), coo_->dims[m], (int)R_, ldr_, seed, (uint64_t)m,
+    factor_init_device(A_[m], Ab_[m], coo_->dims[m], (int)R_, ldr_, seed, (uint64_t)m,
                        stream_);
   ADATM_CUDA(cudaStreamSynchronize(stream_));
 }
@@ -552,9 +561,9 @@ void Engine::set_factors(const double *const *host) {
         for (uint64_t r = R; r < L; ++r) b[i * L + r] = 0.f;
       }
     });
-    ADATM_CUDA(cudaMemcpyAsync(A_[m].get(), b, (size_t)I * ldr_ * sizeof(float),
+    ADATM_CUDA(cudaMemcpyAsync(A_[m], b, (size_t)I * ldr_ * sizeof(float),
                                cudaMemcpyHostToDevice, stream_));
-    if (Ab_[m].get()) to_bf16(A_[m].get(), Ab_[m].get(), I, ldr_, stream_);
+    if (Ab_[m]) to_bf16(A_[m], Ab_[m], I, ldr_, stream_);
   }
   // the copies run on; the staging rows are not reused before they end
   ADATM_CUDA(cudaEventRecord(staged_, stream_));
@@ -567,7 +576,7 @@ void Engine::get_factors(double *const *host) {
   float *buf = staging(total);
   size_t off = 0;
   for (int m = 0; m < coo_->nmodes; ++m) {
-    ADATM_CUDA(cudaMemcpyAsync(buf + off, A_[m].get(), (size_t)coo_->dims[m] * ldr_ * sizeof(float),
+    ADATM_CUDA(cudaMemcpyAsync(buf + off, A_[m], (size_t)coo_->dims[m] * ldr_ * sizeof(float),
                                cudaMemcpyDeviceToHost, stream_));
     off += (size_t)coo_->dims[m] * ldr_;
   }
@@ -593,7 +602,7 @@ void Engine::get_normalized(double *const *host, double *lambda) {
   double *lam = diag + (size_t)N * R_ * R_;
   size_t off = 0;
   for (int m = 0; m < N; ++m) {
-    ADATM_CUDA(cudaMemcpyAsync(buf + off, A_[m].get(), (size_t)coo_->dims[m] * ldr_ * sizeof(float),
+    ADATM_CUDA(cudaMemcpyAsync(buf + off, A_[m], (size_t)coo_->dims[m] * ldr_ * sizeof(float),
                                cudaMemcpyDeviceToHost, stream_));
     ADATM_CUDA(cudaMemcpyAsync(diag + (size_t)m * R_ * R_, G_[m].get(), R_ * R_ * sizeof(double),
                                cudaMemcpyDeviceToHost, stream_));
@@ -638,7 +647,7 @@ double Engine::sweep_download(double *const *host, double *lambda) {
   size_t off = 0;
   for (int m = 0; m < N; ++m) {
     ADATM_CUDA(cudaStreamWaitEvent(copy_, updated_[m], 0));
-    ADATM_CUDA(cudaMemcpyAsync(buf + off, A_[m].get(), (size_t)coo_->dims[m] * ldr_ * sizeof(float),
+    ADATM_CUDA(cudaMemcpyAsync(buf + off, A_[m], (size_t)coo_->dims[m] * ldr_ * sizeof(float),
                                cudaMemcpyDeviceToHost, copy_));
     ADATM_CUDA(cudaMemcpyAsync(diag + (size_t)m * R_ * R_, G_[m].get(), R_ * R_ * sizeof(double),
                                cudaMemcpyDeviceToHost, copy_));
@@ -687,7 +696,7 @@ void Engine::get_lambda(double *host) const {
 
 void Engine::als_begin() {
   for (int m = 0; m < coo_->nmodes; ++m)
-    gram(A_[m].get(), coo_->dims[m], (int)R_, ldr_, G_[m].get(), w_, stream_,
+    gram(A_[m], coo_->dims[m], (int)R_, ldr_, G_[m].get(), w_, stream_,
          opt_.factor_type == FactorType::BF16);
   if (!ttnorm_ready_) {
     frob_sq(csf_[0]->vals64.get(), coo_->nnz, w_, stream_);
@@ -710,7 +719,7 @@ void Engine::sweep_eager() {
     ADATM_CUDA(cudaEventRecord(join_, side_));
     mttkrp_as(m, M_.get(), sweep_type(m));
     ADATM_CUDA(cudaStreamWaitEvent(stream_, join_, 0));
-    update_factor(M_.get(), coo_->dims[m], A_[m].get(), Ab_[m].get(), G_[m].get(), m == N - 1, w_,
+    update_factor(M_.get(), coo_->dims[m], A_[m], Ab_[m], G_[m].get(), m == N - 1, w_,
                   stream_);
     // mode m's rows and Gram are final for this sweep, so a download may
     // start here: an event node when the sweep is being captured (the
@@ -736,7 +745,7 @@ void Engine::update_from(int mode, const double *dev_M) {
   GramSet gs;
   for (int m = 0; m < kMaxModes; ++m) gs.G[m] = m < N ? G_[m].get() : nullptr;
   gram_inverse(gs, mode, w_, stream_);
-  update_factor(dev_M, coo_->dims[mode], A_[mode].get(), Ab_[mode].get(), G_[mode].get(),
+  update_factor(dev_M, coo_->dims[mode], A_[mode], Ab_[mode], G_[mode].get(),
                 mode == N - 1, w_, stream_);
   ADATM_CUDA(cudaStreamSynchronize(stream_));
 }

@@ -15,17 +15,17 @@ namespace adatm {
 
 struct EngineOptions {
   FactorType factor_type = FactorType::F32;
-  uint32_t chunk_leaf = 256;  // source units per chunk (one warp), nonzero sources
-  uint32_t chunk_rows = 128;  // source units per chunk (one warp), memo-row sources
+  uint32_t chunk_leaf = 0;  // source units per chunk, nonzero sources (0 = by size)
+  uint32_t chunk_rows = 0;  // source units per chunk, memo-row sources (0 = by size)
   int max_iters = 1024;       // capacity of the device fit trace
   // contraction walks as a resident grid whose warps claim chunks (fastest
   // for one tensor on the device); off, one chunk per warp, so the blocks of
   // walks running side by side on other streams interleave
   bool resident_grid = true;
-  // walkers per warp in the contraction source loop (0 = default_walkers(R))
+  // walkers per warp of the contractions (0 = default_walkers(R))
   int walkers = 0;
   // unstored levels folded into the contraction source loop (0..2; -1 =
-  // chosen from each tree's fan-out)
+  // as many as each tree's fan-out suggests)
   int fold = -1;
   // no float atomics (the default): every MTTKRP output and memo row is
   // summed in an order fixed by the tree, in FP64 across chunks, so sweeps
@@ -76,7 +76,7 @@ class Engine {
   // ends and normalised on the host while the later modes run. Returns the
   // sweep's fit.
   double sweep_download(double *const *host, double *lambda);
-  float *factor(int m) { return A_[m].get(); }
+  float *factor(int m) { return A_[m]; }
 
   // MTTKRP of `mode` following the plan (tags 0/1/2) into out (dims x ldr
   // FP64, zeroed here). Memo reuse (tag 1) expects the group's memo root to have
@@ -177,8 +177,10 @@ class Engine {
   std::unique_ptr<TreeWalk> walk_[kMaxModes];
   std::unique_ptr<TreeWalk> direct_[kMaxModes];
   std::map<std::tuple<int, int, int>, std::unique_ptr<TreeWalk>> custom_;  // by (mode, tree, tag)
-  DevBuf<float> A_[kMaxModes];
-  DevBuf<__nv_bfloat16> Ab_[kMaxModes];
+  DevBuf<float> factors_;            // every mode's rows, mode after mode
+  DevBuf<__nv_bfloat16> factors16_;  // and their BF16 copies (BF16 engines)
+  float *A_[kMaxModes] = {};
+  __nv_bfloat16 *Ab_[kMaxModes] = {};
   DevBuf<double> G_[kMaxModes];
   DevBuf<double> M_;
   AlsWork w_;

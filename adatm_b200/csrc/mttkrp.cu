@@ -14,13 +14,13 @@ struct WalkArgs {
   uint32_t chunk, nchunks;
   uint64_t nunits;
   uint64_t nfibs[kMaxModes];
+  uint64_t dims[kMaxModes];    // rows of each level's factor
   const uint32_t *fptr[kMaxModes];
   const uint32_t *fids[kMaxModes];
   const float *vals;
   const float *src_rows;       // memo rows of the source level (S < N-1)
   const uint32_t *src_ids;     // fids of the source level
   const uint8_t *src_cd;       // close depths of the source level (S >= 1)
-  const void *U_src;           // factor rows of the source level
   const void *U[kMaxModes];
   float *store[kMaxModes];
   double *out;                 // MTTKRP output rows (FP64 sums)
@@ -29,8 +29,7 @@ struct WalkArgs {
   const uint8_t *hot_slot;     // scatter: slot of an output row summed per block, 0xFF = none
   const uint32_t *hot_rows;    // scatter: output row of each slot
   int nhot;
-  // deterministic contraction: instead of atomics, the partial sums of the
-  // nodes a chunk boundary cuts go to per-chunk rows (head: the node that
+  // contraction: the partial sums of the nodes a chunk boundary cuts go to per-chunk rows (head: the node that
   // began before the chunk and closes in it; tail: the node open at its
   // end), summed later in chunk order; span_lev[l] is level l's slot
   // (-1 = none)
@@ -46,25 +45,11 @@ __device__ __forceinline__ float *span_row(const WalkArgs &a, uint32_t c, int l,
 
 constexpr int kHotRows = 32;     // output rows summed per block, at most
 constexpr uint32_t kHotMin = 32768;  // units that must hit a row to make it one
+constexpr uint32_t kScatterChunk = 128;  // rows per warp of a contraction's scatter
 constexpr uint64_t kHotScanRows = 1ull << 24;  // output rows the hot-row search examines, at most
 
-// ---------------------------------------------------------------------------
-// Warp-uniform tree walk.
-//
-// One warp walks one chunk of consecutive source units; its 32 lanes split
-// the R columns (V = 1, 2 or 4 columns per lane), so every lane follows the
-// same control flow and each factor-row gather is one coalesced access. Units
-// go in batches of 32 (one per lane for the index loads): the batch's factor
-// rows are gathered with many loads in flight, then summed in order into the
-// open node of level S-1. Where a node closes is read from the tree's close
-// depths (no fptr traffic): a unit with close depth c closes its ancestors at
-// levels S-1 .. S-c. The nodes of level S-1 that close in the batch become
-// the items of the next level up -- their sums sit in shared memory, are
-// multiplied by their own factor rows and summed into level S-2 nodes in the
-// same way -- until level d, where completed nodes go to the output.
-// ---------------------------------------------------------------------------
-constexpr int kWarps = 8;   // warps (chunks) per block
-constexpr int kBatch = 32;  // source units per batch
+constexpr int kWarps = 8;   // warps per block
+constexpr int kBatch = 32;  // units per batch of a scatter or pull warp
 
 template <int V>
 struct alignas(sizeof(float) * V) fv {
@@ -78,28 +63,31 @@ __device__ __forceinline__ fv<V> fv_fill(float s) {
   for (int i = 0; i < V; ++i) r.x[i] = s;
   return r;
 }
-template <int V>
-__device__ __forceinline__ void fv_axpy(fv<V> &acc, float s, const fv<V> &b) {
-#pragma unroll
-  for (int i = 0; i < V; ++i) acc.x[i] = fmaf(s, b.x[i], acc.x[i]);
+// Pairs of columns go through the packed FP32 instructions (one issue slot
+// for two products; each is rounded as its scalar form is).
+__device__ __forceinline__ uint64_t pack2(float x, float y) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
 }
-template <int V>
-__device__ __forceinline__ void fv_fma(fv<V> &acc, const fv<V> &a, const fv<V> &b) {
-#pragma unroll
-  for (int i = 0; i < V; ++i) acc.x[i] = fmaf(a.x[i], b.x[i], acc.x[i]);
+__device__ __forceinline__ void unpack2(uint64_t p, float &x, float &y) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(p));
 }
 template <int V>
 __device__ __forceinline__ fv<V> fv_mul(const fv<V> &a, const fv<V> &b) {
   fv<V> r;
+  if constexpr (V == 1) {
+    r.x[0] = a.x[0] * b.x[0];
+  } else {
 #pragma unroll
-  for (int i = 0; i < V; ++i) r.x[i] = a.x[i] * b.x[i];
-  return r;
-}
-template <int V>
-__device__ __forceinline__ fv<V> fv_scale(float s, const fv<V> &a) {
-  fv<V> r;
-#pragma unroll
-  for (int i = 0; i < V; ++i) r.x[i] = s * a.x[i];
+    for (int i = 0; i < V; i += 2) {
+      uint64_t t;
+      asm("mul.rn.f32x2 %0, %1, %2;"
+          : "=l"(t)
+          : "l"(pack2(a.x[i], a.x[i + 1])), "l"(pack2(b.x[i], b.x[i + 1])));
+      unpack2(t, r.x[i], r.x[i + 1]);
+    }
+  }
   return r;
 }
 
@@ -166,34 +154,6 @@ __device__ __forceinline__ fv<V> ld_rows(const float *base, uint64_t row, int ld
   return r;
 }
 
-template <int V>
-__device__ __forceinline__ void st_rows(float *base, uint64_t row, int ldr, int col, const fv<V> &v,
-                                        bool act) {
-  if (!act) return;
-  float *p = base + row * (uint64_t)ldr + col;
-  if constexpr (V == 1) {
-    *p = v.x[0];
-  } else if constexpr (V == 2) {
-    *reinterpret_cast<float2 *>(p) = make_float2(v.x[0], v.x[1]);
-  } else {
-    *reinterpret_cast<float4 *>(p) = make_float4(v.x[0], v.x[1], v.x[2], v.x[3]);
-  }
-}
-
-template <int V>
-__device__ __forceinline__ void red_rows(float *base, uint64_t row, int ldr, int col, const fv<V> &v,
-                                         bool act) {
-  if (!act) return;
-  float *p = base + row * (uint64_t)ldr + col;
-  if constexpr (V == 1) {
-    atomicAdd(p, v.x[0]);
-  } else if constexpr (V == 2) {
-    atomicAdd(reinterpret_cast<float2 *>(p), make_float2(v.x[0], v.x[1]));
-  } else {
-    atomicAdd(reinterpret_cast<float4 *>(p), make_float4(v.x[0], v.x[1], v.x[2], v.x[3]));
-  }
-}
-
 // FP64 output rows: the MTTKRP sums of a row can come from millions of
 // units (a skewed slice), and FP32 sums of that many partials lose several
 // digits; outputs are stored and added in FP64.
@@ -212,32 +172,22 @@ __device__ __forceinline__ void st_out(double *base, uint64_t row, int ldr, int 
   }
 }
 
-template <int V>
-__device__ __forceinline__ void red_out(double *base, uint64_t row, int ldr, int col, const fv<V> &v,
-                                        bool act) {
-  if (!act) return;
-  double *p = base + row * (uint64_t)ldr + col;
-#pragma unroll
-  for (int i = 0; i < V; ++i) atomicAdd(p + i, (double)v.x[i]);
-}
-
 // Factor-row gathers through a per-lane base pointer (the lane's first
 // column) and a byte stride, so an address is one wide multiply-add.
 template <int V, FactorType FT>
 struct RowSrc {
   const char *base = nullptr;
   uint32_t stride = 0;
+  RowSrc() = default;
   // Lanes past the rank read column 0 (their results are never stored).
   __device__ __forceinline__ RowSrc(const void *U, int ldr, int col, bool act) {
     constexpr int esz = FT == FactorType::F32 ? 4 : 2;
     base = static_cast<const char *>(U) + (size_t)(act ? col : 0) * esz;
     stride = (uint32_t)ldr * esz;
   }
-  // Row `row`, or row 0 when !on: the load is always issued at a valid
-  // address, so no branch splits a batch of loads.
-  __device__ __forceinline__ fv<V> load(uint32_t row, bool on) const {
+  __device__ __forceinline__ fv<V> load(uint32_t row) const {
     fv<V> r;
-    const char *p = base + (size_t)(on ? row : 0u) * stride;
+    const char *p = base + (size_t)row * stride;
     if constexpr (FT == FactorType::F32) {
       if constexpr (V == 1) {
         r.x[0] = __ldg(reinterpret_cast<const float *>(p));
@@ -273,369 +223,487 @@ struct RowSrc {
   }
 };
 
-// Shared memory of one contraction warp: kBatch item rows and one row per
-// level 0..N-2 -- the prefix P_l = U_0[node_0] * ... * U_l[node_l] for l < d,
-// the open node's partial sum (carry) for d <= l < S; the two ranges never
-// overlap -- all in fv<V> slots of 32 lanes; then the batch's (id, value)
-// (and parent) words and a 32-word exchange buffer.
+// V columns as packed pairs (one register pair for two FP32 columns), the
+// form the contraction keeps its rows in: no moves between loads and the
+// packed products.
 template <int V>
-__host__ __device__ constexpr size_t contract_warp_smem(int N) {
-  return (size_t)(kBatch + N - 1) * 32 * sizeof(fv<V>) +
-         (kBatch + kBatch / 16) * sizeof(uint4) + kBatch * sizeof(uint32_t);
-}
-// Staging slot of batch unit k: one spare uint4 every 16 units, so the two
-// or four walkers of a warp reading units 16 apart hit different banks.
-__device__ __forceinline__ int ustage_slot(int k) { return k + (k >> 4); }
+struct alignas(4 * V) Row {
+  uint64_t w[V / 2];
+};
+template <>
+struct alignas(4) Row<1> {
+  float w;
+};
 template <int V>
-constexpr size_t contract_smem(int N) {
-  return (size_t)kWarps * contract_warp_smem<V>(N);
-}
-
-// Recompute the prefix rows of levels lo..hi-1 from the node indices (lane l
-// of nodeL holds the node of level l).
-template <int V, FactorType FT>
-__device__ __noinline__ void refresh_prefix(const WalkArgs &a, fv<V> *pre, uint32_t nodeL, int lo,
-                                            int hi, int col, bool act, int lane) {
-  for (int l = lo; l < hi; ++l) {
-    const uint32_t n = __shfl_sync(~0u, nodeL, l);
-    const bool valid = (uint64_t)n < a.nfibs[l];
-    const uint32_t f = valid ? __ldg(a.fids[l] + n) : 0u;
-    const fv<V> row = ld_factor<V, FT>(a.U[l], f, a.ldr, col, act && valid);
-    pre[l * 32 + lane] = l == 0 ? row : fv_mul(pre[(l - 1) * 32 + lane], row);
+__device__ __forceinline__ Row<V> row_zero() {
+  Row<V> r;
+  if constexpr (V == 1) {
+    r.w = 0.f;
+  } else {
+#pragma unroll
+    for (int i = 0; i < V / 2; ++i) r.w[i] = 0ull;
   }
-}
-
-// Levels lo..hi-1 move on to their next node (their nodes closed); their
-// prefix rows are recomputed. Returns the updated per-lane node register.
-template <int V, FactorType FT>
-__device__ __noinline__ uint32_t advance_prefix(const WalkArgs &a, fv<V> *pre, uint32_t nodeL,
-                                                int lo, int hi, int col, bool act, int lane) {
-  if (lane >= lo && lane < hi) nodeL += 1;
-  if (lo < hi && (uint64_t)__shfl_sync(~0u, nodeL, lo) < a.nfibs[lo])
-    refresh_prefix<V, FT>(a, pre, nodeL, lo, hi, col, act, lane);
-  return nodeL;
-}
-
-// Compaction of per-lane values onto the set bits of m: lane i gets the
-// value of the lane holding the i-th set bit (i < popc(m)), else 0.
-__device__ __forceinline__ uint32_t compact_bits(uint32_t m, uint32_t value, uint32_t *xbuf, int lane) {
-  if ((m >> lane) & 1u) xbuf[__popc(m & lanemask_lt())] = value;
-  __syncwarp();
-  const uint32_t r = lane < __popc(m) ? xbuf[lane] : 0u;
-  __syncwarp();
   return r;
 }
-
-// Contraction (S > d).
-//
-// The source units of a batch are summed into the open node of level S-1
-// (carry `acc`, in registers); the level-(S-1) nodes that close become the
-// batch's items. The level loop then takes the items up one level at a time
-// -- memo stores, the items' own factor rows, carries of the levels above in
-// shared memory -- until level d. Resident blocks per SM follow the shared
-// memory a block takes (4 at V = 1, so at most 64 registers per thread).
 template <int V>
-constexpr int contract_min_blocks() {
-  return V == 1 ? 4 : (V == 2 ? 2 : 1);
+__device__ __forceinline__ fv<V> row_values(const Row<V> &r) {
+  fv<V> f;
+  if constexpr (V == 1) {
+    f.x[0] = r.w;
+  } else {
+#pragma unroll
+    for (int i = 0; i < V / 2; ++i) unpack2(r.w[i], f.x[2 * i], f.x[2 * i + 1]);
+  }
+  return f;
+}
+template <int V>
+__device__ __forceinline__ Row<V> row_mul(const Row<V> &a, const Row<V> &b) {
+  Row<V> r;
+  if constexpr (V == 1) {
+    r.w = a.w * b.w;
+  } else {
+#pragma unroll
+    for (int i = 0; i < V / 2; ++i)
+      asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.w[i]) : "l"(a.w[i]), "l"(b.w[i]));
+  }
+  return r;
+}
+template <int V>
+__device__ __forceinline__ Row<V> row_add(const Row<V> &a, const Row<V> &b) {
+  Row<V> r;
+  if constexpr (V == 1) {
+    r.w = a.w + b.w;
+  } else {
+#pragma unroll
+    for (int i = 0; i < V / 2; ++i)
+      asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.w[i]) : "l"(a.w[i]), "l"(b.w[i]));
+  }
+  return r;
+}
+template <int V>
+__device__ __forceinline__ void row_fma(Row<V> &acc, const Row<V> &a, const Row<V> &b) {
+  if constexpr (V == 1) {
+    acc.w = fmaf(a.w, b.w, acc.w);
+  } else {
+#pragma unroll
+    for (int i = 0; i < V / 2; ++i)
+      asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc.w[i]) : "l"(a.w[i]), "l"(b.w[i]));
+  }
+}
+// A factor row as it is loaded: FP32 columns, or BF16 pairs.
+template <int V, FactorType FT>
+struct RawRow {
+  Row<V> r;
+};
+template <int V>
+struct RawRow<V, FactorType::BF16> {
+  uint32_t w[(V + 1) / 2];
+};
+template <int V, FactorType FT>
+__device__ __forceinline__ Row<V> raw_row(const RawRow<V, FT> &a) {
+  if constexpr (FT == FactorType::F32) {
+    return a.r;
+  } else {
+    // a BF16 value is the upper half of its FP32 value
+    Row<V> r;
+    if constexpr (V == 1) {
+      r.w = __uint_as_float(a.w[0] << 16);
+    } else {
+#pragma unroll
+      for (int i = 0; i < V / 2; ++i)
+        r.w[i] = pack2(__uint_as_float(a.w[i] << 16), __uint_as_float(a.w[i] & 0xFFFF0000u));
+    }
+    return r;
+  }
+}
+// Loaded where on != 0, without a branch; elsewhere the row keeps its value.
+template <int V, FactorType FT>
+__device__ __forceinline__ void ld_row_if(RawRow<V, FT> &a, const char *p, uint32_t on) {
+  if constexpr (FT == FactorType::F32) {
+    if constexpr (V == 1)
+      asm("{\n.reg .pred q;\nsetp.ne.u32 q, %2, 0;\n@q ld.global.nc.f32 %0, [%1];\n}"
+          : "+f"(a.r.w)
+          : "l"(p), "r"(on));
+    else if constexpr (V == 2)
+      asm("{\n.reg .pred q;\nsetp.ne.u32 q, %2, 0;\n@q ld.global.nc.b64 %0, [%1];\n}"
+          : "+l"(a.r.w[0])
+          : "l"(p), "r"(on));
+    else
+      asm("{\n.reg .pred q;\nsetp.ne.u32 q, %3, 0;\n@q ld.global.nc.v2.b64 {%0, %1}, [%2];\n}"
+          : "+l"(a.r.w[0]), "+l"(a.r.w[1])
+          : "l"(p), "r"(on));
+  } else {
+    if constexpr (V == 1)
+      asm("{\n.reg .pred q;\n.reg .b16 h;\nsetp.ne.u32 q, %2, 0;\n@q ld.global.nc.b16 h, [%1];\n"
+          "@q cvt.u32.u16 %0, h;\n}"
+          : "+r"(a.w[0])
+          : "l"(p), "r"(on));
+    else if constexpr (V == 2)
+      asm("{\n.reg .pred q;\nsetp.ne.u32 q, %2, 0;\n@q ld.global.nc.b32 %0, [%1];\n}"
+          : "+r"(a.w[0])
+          : "l"(p), "r"(on));
+    else
+      asm("{\n.reg .pred q;\nsetp.ne.u32 q, %3, 0;\n@q ld.global.nc.v2.b32 {%0, %1}, [%2];\n}"
+          : "+r"(a.w[0]), "+r"(a.w[1])
+          : "l"(p), "r"(on));
+  }
+}
+template <int V, FactorType FT>
+__device__ __forceinline__ void raw_zero(RawRow<V, FT> &a) {
+  if constexpr (FT == FactorType::F32) {
+    a.r = row_zero<V>();
+  } else {
+#pragma unroll
+    for (int i = 0; i < (V + 1) / 2; ++i) a.w[i] = 0u;
+  }
+}
+template <int V, FactorType FT>
+__device__ __forceinline__ void ld_row(RawRow<V, FT> &a, const char *p) {
+  if constexpr (FT == FactorType::F32) {
+    if constexpr (V == 1)
+      asm("ld.global.nc.f32 %0, [%1];" : "=f"(a.r.w) : "l"(p));
+    else if constexpr (V == 2)
+      asm("ld.global.nc.b64 %0, [%1];" : "=l"(a.r.w[0]) : "l"(p));
+    else
+      asm("ld.global.nc.v2.b64 {%0, %1}, [%2];" : "=l"(a.r.w[0]), "=l"(a.r.w[1]) : "l"(p));
+  } else {
+    if constexpr (V == 1)
+      a.w[0] = __ldg(reinterpret_cast<const unsigned short *>(p));
+    else if constexpr (V == 2)
+      asm("ld.global.nc.b32 %0, [%1];" : "=r"(a.w[0]) : "l"(p));
+    else
+      asm("ld.global.nc.v2.b32 {%0, %1}, [%2];" : "=r"(a.w[0]), "=r"(a.w[1]) : "l"(p));
+  }
+}
+template <int V, FactorType FT>
+__device__ __forceinline__ Row<V> ld_row(const char *p) {
+  RawRow<V, FT> a;
+  ld_row<V, FT>(a, p);
+  return raw_row<V, FT>(a);
+}
+__device__ __forceinline__ const char *row_at(const char *base, uint32_t row, uint32_t stride) {
+  return base + (uint64_t)row * stride;
+}
+// The tree's arrays are read once, in order: a miss brings the next units
+// into L2 as well.
+__device__ __forceinline__ uint32_t ld_stream(const uint32_t *p) {
+  uint32_t v;
+  asm("ld.global.nc.L2::256B.b32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float ld_stream(const float *p) {
+  float v;
+  asm("ld.global.nc.L2::256B.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint32_t ld_stream(const uint8_t *p) {
+  uint32_t v;
+  asm("ld.global.nc.L2::256B.u8 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
 }
 
+// ---------------------------------------------------------------------------
+// Contraction (S > d).
 //
-// FOLD F (levels S-1 .. S-F are not stored and lie below d): the nodes of
-// those levels are not formed. Each unit's product is multiplied by the
-// factor rows of its ancestors at levels S-1 .. S-F (U_{S-1} of the
-// level-(S-1) node holding it, and at F = 2 U_{S-2} of the level-(S-2) node
-// holding that) and summed straight into the open node of level S-1-F, so
-// the batch's items are level-(S-1-F) nodes. The ancestors of a batch's
-// units are consecutive nodes from each level's open node on (a unit's is
-// the open node plus the closes of that level before it), so their ids come
-// with one coalesced load per level. Folding trades one item of level l for
-// one extra gather per unit below it: it pays where levels are hypersparse
-// (few units per node). The sums equal the unfolded ones up to FP32
-// rounding order.
-// WALKERS: the source loop of a batch runs as W walkers of 32/W lanes, each
-// over its own contiguous segment of 32/W units with VW columns per lane, so
-// one warp instruction advances W units. Each walker sums its segment into
-// its own open node; the nodes that close in a walker's segment become items
-// as before, and the segments are joined once per batch: the sum a walker
-// carries past its segment flows into the next walker's first closed node
-// (or on through, when that walker closes none), W - 1 shuffle rounds. The
-// level loop keeps the warp-wide layout (V columns per lane); items and
-// carry rows are plain column-ordered rows in shared memory, so both
-// layouts read them.
-template <int V, int W, int VW, FactorType FT, bool LEAF, int F>
-__global__ void __launch_bounds__(256, contract_min_blocks<V>())
-    k_contract(const __grid_constant__ WalkArgs a) {
-  static_assert(F >= 0 && F <= 2, "folded levels");
-  static_assert(W == 1 || W == 2 || W == 4, "walkers per warp");
-  static_assert((32 / W) * VW <= 32 * V, "a walker's columns must fit the item rows");
-  constexpr int L = 32 / W;        // lanes per walker
-  constexpr int SEG = kBatch / W;  // units per walker per batch
+// A warp runs W independent walkers of L = 32 / W lanes with VW columns per
+// lane; each walker walks its own chunk of consecutive source units, so one
+// warp instruction advances W units and nothing is exchanged between walkers.
+// Where a node closes is read from the tree's close depths (no fptr traffic):
+// a unit with close depth c closes its ancestors at levels S-1 .. S-c.
+//
+// FOLD F (levels S-1 .. S-F are not stored and lie below d; at most
+// kMaxFold): the nodes of those levels are not formed. Each unit's row is
+// multiplied by the factor rows of its ancestors at levels S-1 .. S-F and
+// summed straight into the open node of level top = S-1-F (acc). The
+// ancestors of a batch's units are consecutive nodes from each level's open
+// node on (a unit's is the open node plus the closes of that level before
+// it), so their ids come with one coalesced load per level.
+//
+// A node of level top that closes leaves the unit loop: its sum is stored
+// (memo rows, outputs), or multiplied by its own factor row and added to the
+// open node of the level above, in shared memory, and so on up as far as the
+// unit closes. The sums of the nodes that a chunk boundary cuts go to
+// per-chunk head and tail rows (k_chain_groups adds them).
+//
+// What bounds it: the L1 data pipe and the latency of the gathers behind it,
+// not DRAM. A row of R = 32 columns takes one of its cycles, so a unit takes
+// F + 1, next to about two for the staging and the closes. On the 6th-order
+// Zipf(1.3) tensor at 10.4M nonzeros (R = 32, F = 3) the pipe is busy 71% of
+// the time at 18 warp instructions per nonzero (issue 51%): 0.36 ms, against
+// 0.47 ms and 29 instructions for one walk per warp whose closes went through
+// shared-memory items; the 77.9M-nonzero tensor's three contractions 2.32 /
+// 2.18 / 1.97 ms against 2.62 / 2.43 / 2.23. Measured and not kept: rows of
+// the folded levels kept across units and loaded under a predicate (a load
+// with inactive lanes costs the pipe as much as a full one), one unit in
+// flight with the next one's rows loaded ahead (2.33), three or five blocks
+// per SM (2.46 / 2.48), two walkers of two columns per lane (3.26).
+// ---------------------------------------------------------------------------
+constexpr int kMaxFold = 5;
+
+template <int W>
+struct WalkShape {
+  static constexpr int L = 32 / W;            // lanes per walker
+  static constexpr int B = L < 16 ? 16 : 32;   // units per walker and batch
+  static constexpr int RD = B / L;            // staging rounds per batch
+};
+
+// Shared memory of one warp: the batch's staged units (a uint4 per unit: its
+// row, its parent's row, its value twice, as the packed products take it;
+// the rows of the ancestors further up in X words; its close depth), one
+// spare slot per walker, so that walkers read different banks; the open nodes
+// (a word per lane) and open sums (VW columns per lane) of levels d .. top-1.
+__host__ __device__ constexpr int stage_words(int F) { return F <= 1 ? 0 : (F == 2 ? 1 : (F == 3 ? 2 : 4)); }
+template <int W, int VW, int F>
+__host__ __device__ constexpr size_t contract_warp_smem(int d, int top) {
+  return (size_t)W * (WalkShape<W>::B + 1) * (sizeof(uint4) + stage_words(F) * sizeof(uint32_t)) / 16 * 16 + 16 +
+         (size_t)W * WalkShape<W>::B +
+         (size_t)(top > d ? top - d : 0) * 32 * (sizeof(uint32_t) + VW * sizeof(float));
+}
+
+// What the unit loop reads: factor rows of the source and folded levels lie
+// in one allocation, addressed by row number from its base.
+struct HotArgs {
+  const void *base;             // row 0
+  uint32_t src_row;             // first row of the source level's factor
+  uint32_t fold_row[kMaxFold];  // and of level S-1-f's
+  const uint32_t *fold_ids[kMaxFold];
+  const uint32_t *top_ids;
+  const void *top_rows;         // factor of level top
+  uint32_t top_last;            // its last node
+  float *top_store;             // its memo rows
+  int top_keep;                 // whether its sums are stored or output
+};
+
+template <int W, int VW, FactorType FT, bool LEAF, int F>
+__global__ void __launch_bounds__(256, 4)
+    k_contract(const __grid_constant__ WalkArgs a, const __grid_constant__ HotArgs hot) {
+  static_assert(F >= 0 && F <= kMaxFold, "folded levels");
+  constexpr int L = WalkShape<W>::L, B = WalkShape<W>::B, RD = WalkShape<W>::RD;
+  constexpr uint32_t LM = L == 32 ? 0xFFFFFFFFu : (1u << L) - 1u;
   extern __shared__ __align__(16) unsigned char walk_raw[];
+  const int S = a.S, d = a.d, top = a.S - 1 - F;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  unsigned char *wbase = walk_raw + (size_t)warp * contract_warp_smem<V>(a.N);
-  fv<V> *items = reinterpret_cast<fv<V> *>(wbase);
-  float *items_f = reinterpret_cast<float *>(wbase);  // row j: 32 * V floats
-  fv<V> *carry = items + kBatch * 32;  // rows d..S-1
-  fv<V> *pre = carry;                  // rows 0..d-1
-  uint4 *ustage = reinterpret_cast<uint4 *>(carry + (a.N - 1) * 32);
-  uint32_t *xbuf = reinterpret_cast<uint32_t *>(ustage + kBatch + kBatch / 16);
-  const int col = lane * V;
+  const int wk = lane / L, li = lane % L;
+  unsigned char *wbase = walk_raw + (size_t)warp * contract_warp_smem<W, VW, F>(d, top);
+  constexpr int X = stage_words(F);
+  constexpr size_t kStageBytes =
+      (size_t)W * (B + 1) * (sizeof(uint4) + X * sizeof(uint32_t)) / 16 * 16 + 16;
+  uint4 *const stage = reinterpret_cast<uint4 *>(wbase) + wk * (B + 1);
+  uint32_t *const stage2 =
+      reinterpret_cast<uint32_t *>(reinterpret_cast<uint4 *>(wbase) + W * (B + 1)) + wk * (B + 1) * X;
+  uint8_t *const scd = wbase + kStageBytes + wk * B;
+  // open node and open sum of level l in {d .. top-1}: nodes[l * 32], carry[l * 32]
+  uint32_t *const nodes = reinterpret_cast<uint32_t *>(wbase + kStageBytes + W * B) + lane - d * 32;
+  Row<VW> *const carry =
+      reinterpret_cast<Row<VW> *>(nodes + (top > d ? top : d) * 32 - lane) + lane - d * 32;
+  const int col = li * VW;
   const bool act = col < a.R;
-  const int wk = lane / L;           // this lane's walker
-  const int wcol = (lane % L) * VW;  // its first column in the walker layout
-  const bool wact = wcol < a.R;
-  const int S = a.S, d = a.d;
-  // a resident grid: each warp claims chunks from a counter, the next one
-  // while it walks the current one; without a counter, one chunk per warp
-  const bool claims = a.counter != nullptr;
-  uint32_t claim = claims && lane == 0 ? atomicAdd(a.counter, 1u) : 0u;
-  uint32_t chunk_id = claims ? __shfl_sync(~0u, claim, 0) : blockIdx.x * kWarps + warp;
-  while (chunk_id < a.nchunks) {
-    if (claims && lane == 0) claim = atomicAdd(a.counter, 1u);
-    const uint32_t *sc = a.sched + (size_t)chunk_id * (S + 1);
-    uint32_t nodeL = lane < S ? sc[lane] : 0u;
+  constexpr int esz = FT == FactorType::F32 ? 4 : 2;
+  // row offsets are staged in units of four columns (32 bits number the rows of
+  // any factor that fits the device)
+  constexpr int kUnitShift = FT == FactorType::F32 ? 4 : 3;
+  const uint32_t row_units = (uint32_t)a.ldr / 4u;
+  // lanes past the rank read column 0 (their results are never stored)
+  const uint32_t lane_off = (uint32_t)(act ? col : 0) * esz;
+  const char *rows = static_cast<const char *>(hot.base) + lane_off;
+  asm volatile("" : "+l"(rows));  // kept, not computed again at each load
+  const char *const rows_t = static_cast<const char *>(hot.top_rows) + lane_off;
+  const uint32_t stride = (uint32_t)a.ldr * esz;
+
+  // units whose rows are in flight together: as many as the registers hold
+  constexpr int SB = VW <= 2 ? 4 : (F <= 3 ? 2 : 1);
+  // the first group of W chunks by the warp's place in the grid, the next
+  // ones from a counter (a resident grid), claimed while the current one runs
+  uint32_t group = blockIdx.x * kWarps + warp;
+  const uint32_t ngroups = (a.nchunks + W - 1) / W;
+  while (group < ngroups) {
+    uint32_t claim = 0;
+    if (a.counter != nullptr && lane == 0) claim = atomicAdd(a.counter, 1u);
+    const uint32_t chunk_id = group * W + wk;
+    const bool live = chunk_id < a.nchunks;
+    const uint32_t *sc = a.sched + (size_t)(live ? chunk_id : 0u) * (S + 1);
     uint32_t part = sc[S];
-    uint32_t touched = 0;
-    for (int l = d; l < S - 1; ++l) carry[l * 32 + lane] = fv_fill<V>(0.f);
-    if (d > 0) refresh_prefix<V, FT>(a, pre, nodeL, 0, d, col, act, lane);
-    const RowSrc<VW, FT> Us(a.U_src, a.ldr, wcol, wact);
-    const RowSrc<VW, FT> Up(F >= 1 ? a.U[S - 1] : a.U_src, a.ldr, wcol, wact);
-    const RowSrc<VW, FT> Uq(F >= 2 ? a.U[S - 2] : a.U_src, a.ldr, wcol, wact);
-    const int top = S - 1 - F;  // level whose open node the units feed
-    // open node of level `top` carried in from earlier batches (every walker
-    // holds the same copy)
-    fv<VW> acc = fv_fill<VW>(0.f);
-    // unit rows in flight per lane, never more than the walker's segment:
-    // fewer as each unit gathers more rows (the 64 registers a thread has at
-    // four blocks per SM are the limit; spilling costs more than the extra
-    // load latency exposed)
-    constexpr int SB0 = (F == 2 ? 4 : (F == 1 ? 8 : 16)) / VW;
-    constexpr int SB = SB0 < SEG ? SB0 : SEG;
-    static_assert(SEG % SB == 0, "a walker's segment is a whole number of load groups");
-    const uint64_t u0 = (uint64_t)chunk_id * a.chunk;
-    const uint64_t u1 = min(u0 + a.chunk, a.nunits);
-    for (uint64_t base = u0; base < u1; base += kBatch) {
-      const int cnt = (int)min((uint64_t)kBatch, u1 - base);
-      const bool in = lane < cnt;
-      const uint32_t id = in ? __ldg(a.src_ids + base + lane) : 0u;
-      float v = 0.f;
-      if constexpr (LEAF) v = in ? __ldg(a.vals + base + lane) : 0.f;
-      const uint32_t cd = in ? (uint32_t)__ldg(a.src_cd + base + lane) : 0u;
-      const uint32_t M = __ballot_sync(~0u, cd >= 1u);
-      uint32_t pfid = 0u, qfid = 0u, M2 = 0u;
-      if constexpr (F >= 1) {
-        // unit lane sits in level-(S-1) node first + (closes before it)
-        const uint64_t pn = (uint64_t)__shfl_sync(~0u, nodeL, S - 1) + __popc(M & lanemask_lt());
-        if (in && pn < a.nfibs[S - 1]) pfid = __ldg(a.fids[S - 1] + pn);
+    uint32_t nt = sc[top];
+    uint32_t nf[F >= 1 ? F : 1];  // open nodes of the folded levels
+#pragma unroll
+    for (int f = 0; f < F; ++f) nf[f] = sc[S - 1 - f];
+    for (int l = d; l < top; ++l) {
+      nodes[l * 32] = sc[l];
+      carry[l * 32] = row_zero<VW>();
+    }
+    uint32_t idt = __ldg(hot.top_ids + nt);  // the open level-top node's id
+    Row<VW> acc = row_zero<VW>();
+    // The sum x of a closed node: to its memo row, or, if it began before the
+    // chunk, to the chunk's head row; at the root output, to its output row.
+    auto keep = [&](int l, float *store, uint32_t n, uint32_t id, const Row<VW> &x) {
+      if ((part >> l) & 1u) {
+        part &= ~(1u << l);
+        if (act) *reinterpret_cast<Row<VW> *>(span_row(a, chunk_id, l, 0) + col) = x;
+      } else {
+        if (store != nullptr && act) *reinterpret_cast<Row<VW> *>(store + (size_t)n * (uint32_t)a.ldr + col) = x;
+        if (l == 0 && a.out != nullptr) st_out<VW>(a.out, id, a.ldr, col, row_values(x), act);
       }
-      if constexpr (F >= 2) {
-        // and in level-(S-2) node first + (level-(S-2) closes before it)
-        M2 = __ballot_sync(~0u, cd >= 2u);
-        const uint64_t qn = (uint64_t)__shfl_sync(~0u, nodeL, S - 2) + __popc(M2 & lanemask_lt());
-        if (in && qn < a.nfibs[S - 2]) qfid = __ldg(a.fids[S - 2] + qn);
+    };
+    // A unit closes level top and `more` levels above it.
+    auto close = [&](uint32_t more) {
+      Row<VW> x = acc;
+      acc = row_zero<VW>();
+      const uint32_t id = idt;
+      if (hot.top_keep) keep(top, hot.top_store, nt, id, x);
+      ++nt;
+      if (top == d) {
+        if (d == 0) idt = __ldg(hot.top_ids + min(nt, hot.top_last));
+        return;
       }
-      // closes of level `top`
-      const uint32_t Mc = F == 0 ? M : (F == 1 ? __ballot_sync(~0u, cd >= 2u) : __ballot_sync(~0u, cd >= 3u));
-      ustage[ustage_slot(lane)] = make_uint4(id, __float_as_uint(v), pfid, qfid);
+      Row<VW> c = carry[(top - 1) * 32];
+      const Row<VW> row = ld_row<VW, FT>(row_at(rows_t, id, stride));
+      idt = __ldg(hot.top_ids + min(nt, hot.top_last));
+      row_fma(c, x, row);
+      int l = top - 1;
+      for (; more != 0u; --more) {
+        carry[l * 32] = row_zero<VW>();
+        const uint32_t n = nodes[l * 32];
+        nodes[l * 32] = n + 1u;
+        const uint32_t up = __ldg(a.fids[l] + n);
+        if (a.span_lev[l] >= 0) keep(l, a.store[l], n, up, c);
+        if (l == d) return;
+        x = c;
+        --l;
+        c = carry[l * 32];
+        row_fma(c, x, ld_row<VW, FT>(row_at(static_cast<const char *>(a.U[l + 1]) + lane_off, up, stride)));
+      }
+      carry[l * 32] = c;
+    };
+    uint32_t lastcd = 0u;
+    const uint32_t u0 = live ? chunk_id * a.chunk : 0u;  // (units are numbered in 32 bits)
+    const uint32_t left0 = live ? min(a.chunk, (uint32_t)a.nunits - u0) : 0u;
+    for (uint32_t b0 = 0; b0 < a.chunk; b0 += B) {
+      const int cnt = left0 > b0 ? (int)min((uint32_t)B, left0 - b0) : 0;
+      if (!__any_sync(~0u, cnt > 0)) break;
+      const uint32_t base = u0 + b0;
+      // stage the batch; mt: the units that close level top
+      uint32_t mt = 0u;
+      {
+        uint32_t id[RD], cd[RD], anc[RD][5];
+        float v[RD];
+#pragma unroll
+        for (int r = 0; r < RD; ++r) {
+          const int j = r * L + li;
+          const bool in = j < cnt;
+          id[r] = in ? ld_stream(a.src_ids + (base + j)) : 0u;
+          v[r] = 0.f;
+          if constexpr (LEAF) v[r] = in ? ld_stream(a.vals + (base + j)) : 0.f;
+          cd[r] = in ? ld_stream(a.src_cd + (base + j)) : 0u;
+        }
+#pragma unroll
+        for (int r = 0; r < RD; ++r) {
+          const bool in = r * L + li < cnt;
+          const uint32_t lt = (1u << li) - 1u;
+#pragma unroll
+          for (int f = 0; f < 5; ++f) {
+            anc[r][f] = 0u;
+            if (f < F) {
+              const uint32_t m = (__ballot_sync(~0u, cd[r] >= (uint32_t)(f + 1)) >> (wk * L)) & LM;
+              uint32_t &n = nf[f < F ? f : 0];
+              if (in) anc[r][f] = (ld_stream(hot.fold_ids[f] + (n + __popc(m & lt))) + hot.fold_row[f]) * row_units;
+              n += __popc(m);
+            }
+          }
+          mt |= ((__ballot_sync(~0u, cd[r] >= (uint32_t)(F + 1)) >> (wk * L)) & LM) << (r * L);
+        }
+#pragma unroll
+        for (int r = 0; r < RD; ++r) {
+          const int j = r * L + li;
+          const uint32_t vb = __float_as_uint(v[r]);
+          stage[j] = make_uint4((id[r] + hot.src_row) * row_units, anc[r][0], vb, vb);
+          if constexpr (X >= 1) stage2[j * X] = anc[r][1];
+          if constexpr (X >= 2) stage2[j * X + 1] = anc[r][2];
+          if constexpr (X >= 4) {
+            stage2[j * X + 2] = anc[r][3];
+            stage2[j * X + 3] = anc[r][4];
+          }
+          scd[j] = (uint8_t)cd[r];
+        }
+      }
       __syncwarp();
-      // this walker's units are k_lo .. k_lo + SEG - 1: its closes, and the
-      // item index of its first close
-      const int k_lo = wk * SEG;
-      const uint32_t below = k_lo == 0 ? 0u : (0xFFFFFFFFu >> (32 - k_lo));
-      const uint32_t Mw = Mc & ((0xFFFFFFFFu >> (32 - SEG)) << k_lo);
-      const int j0 = __popc(Mc & below);
-      int j = j0;
-      fv<VW> wacc = W == 1 ? acc : fv_fill<VW>(0.f);
-      auto emit = [&](const fv<VW> &x) {
-        *reinterpret_cast<fv<VW> *>(items_f + (size_t)j * 32 * V + wcol) = x;
-        ++j;
-      };
+      // the unit loop, the same for every lane; only a close is a walker's own
+      const uint32_t any = __reduce_or_sync(~0u, mt);
+      const char *mrow = nullptr;
+      if constexpr (!LEAF)
+        mrow = reinterpret_cast<const char *>(a.src_rows + (uint64_t)base * (uint32_t)a.ldr + (act ? col : 0));
       auto run = [&](auto full) {
         constexpr bool FULL = decltype(full)::value;
-#pragma unroll
-        for (int q0 = 0; q0 < SEG; q0 += SB) {
-          if (!FULL && k_lo + q0 >= cnt) break;
-          fv<VW> g[SB];
-          fv<VW> h[F >= 1 ? SB : 1];
-          fv<VW> h2[F >= 2 ? SB : 1];
-          fv<VW> m[LEAF ? 1 : SB];
-          float vv[LEAF ? SB : 1];
+#pragma unroll 1
+        for (int k = 0; k < B; k += SB) {
+          if (!FULL && !__any_sync(~0u, k < cnt)) break;
+          RawRow<VW, FT> g[SB], t[SB][F >= 1 ? F : 1];
+          RawRow<VW, FactorType::F32> m[LEAF ? 1 : SB];
+          uint64_t v[LEAF ? SB : 1];
 #pragma unroll
           for (int q = 0; q < SB; ++q) {
-            const int k = k_lo + q0 + q;
-            // lanes past the rank read column 0 through Us's base, so only
-            // the units past the batch need the row-0 substitute
-            const bool ok = FULL || k < cnt;
-            const uint4 e = ustage[ustage_slot(k)];
-            g[q] = Us.load(e.x, ok);
-            if constexpr (F >= 1) h[q] = Up.load(e.z, ok);
-            if constexpr (F >= 2) h2[q] = Uq.load(e.w, ok);
-            if constexpr (LEAF) vv[q] = __uint_as_float(e.y);
-            if constexpr (!LEAF) m[q] = ld_rows<VW>(a.src_rows, base + k, a.ldr, wcol, ok && wact);
+            // units past the walker's last are staged as row 0 and not added
+            const uint4 e = stage[k + q];
+            ld_row<VW, FT>(g[q], rows + ((uint64_t)e.x << kUnitShift));
+            if constexpr (F >= 1) ld_row<VW, FT>(t[q][0], rows + ((uint64_t)e.y << kUnitShift));
+            const uint32_t *e2 = stage2 + (k + q) * X;
+            if constexpr (F >= 2) ld_row<VW, FT>(t[q][1], rows + ((uint64_t)e2[0] << kUnitShift));
+            if constexpr (F >= 3) ld_row<VW, FT>(t[q][2], rows + ((uint64_t)e2[1] << kUnitShift));
+            if constexpr (F >= 4) ld_row<VW, FT>(t[q][3], rows + ((uint64_t)e2[2] << kUnitShift));
+            if constexpr (F >= 5) ld_row<VW, FT>(t[q][4], rows + ((uint64_t)e2[3] << kUnitShift));
+            if constexpr (LEAF) {
+              v[q] = pack2(__uint_as_float(e.z), __uint_as_float(e.w));
+            } else {
+              raw_zero<VW, FactorType::F32>(m[q]);
+              if (FULL || k + q < cnt) ld_row<VW, FactorType::F32>(m[q], mrow);
+              mrow += (uint32_t)a.ldr * 4u;
+            }
           }
 #pragma unroll
           for (int q = 0; q < SB; ++q) {
-            const int k = k_lo + q0 + q;
-            if (FULL || k < cnt) {
-              if constexpr (F >= 1) {
-                fv<VW> x = LEAF ? fv_scale(vv[LEAF ? q : 0], g[q]) : fv_mul(m[LEAF ? 0 : q], g[q]);
-                if constexpr (F >= 2) {
-                  x = fv_mul(x, h[q]);
-                  fv_fma(wacc, x, h2[F >= 2 ? q : 0]);
-                } else {
-                  fv_fma(wacc, x, h[F >= 1 ? q : 0]);
-                }
-              } else if constexpr (LEAF) {
-                fv_axpy(wacc, vv[LEAF ? q : 0], g[q]);
-              } else {
-                fv_fma(wacc, m[LEAF ? 0 : q], g[q]);
-              }
-              if ((Mw >> k) & 1u) {
-                emit(wacc);
-                wacc = fv_fill<VW>(0.f);
-              }
+            Row<VW> x = raw_row<VW, FT>(g[q]);
+#pragma unroll
+            for (int f = 0; f < F; ++f) x = row_mul(x, raw_row<VW, FT>(t[q][f]));
+            Row<VW> y;
+            if constexpr (!LEAF) {
+              y = raw_row<VW, FactorType::F32>(m[q]);
+            } else if constexpr (VW == 1) {
+              float lo, hi;
+              unpack2(v[q], lo, hi);
+              y.w = lo;
+            } else {
+#pragma unroll
+              for (int i = 0; i < VW / 2; ++i) y.w[i] = v[q];
+            }
+            if (FULL || k + q < cnt) row_fma(acc, x, y);
+            if ((any >> (k + q)) & 1u) {
+              if ((mt >> (k + q)) & 1u) close((uint32_t)scd[k + q] - (uint32_t)(F + 1));
+              __syncwarp();
             }
           }
         }
       };
-      if (cnt == kBatch) run(std::true_type{});
+      if (__all_sync(~0u, cnt == B)) run(std::true_type{});
       else run(std::false_type{});
-      if constexpr (W == 1) {
-        acc = wacc;
-      } else {
-        // join the segments: the inflow of walker w is what walker w-1
-        // carries past its segment (the carry-in for walker 0)
-        const bool hc = Mw != 0u;
-        fv<VW> inflow = acc, out;
-#pragma unroll
-        for (int i = 0; i < VW; ++i) out.x[i] = hc ? wacc.x[i] : inflow.x[i] + wacc.x[i];
-#pragma unroll
-        for (int r = 0; r + 1 < W; ++r) {
-#pragma unroll
-          for (int i = 0; i < VW; ++i) {
-            const float up = __shfl_up_sync(~0u, out.x[i], L);
-            if (wk == r + 1) {
-              inflow.x[i] = up;
-              out.x[i] = hc ? wacc.x[i] : up + wacc.x[i];
-            }
-          }
-        }
-        if (hc) {
-          fv<VW> *first = reinterpret_cast<fv<VW> *>(items_f + (size_t)j0 * 32 * V + wcol);
-          fv<VW> t = *first;
-#pragma unroll
-          for (int i = 0; i < VW; ++i) t.x[i] += inflow.x[i];
-          *first = t;
-        }
-#pragma unroll
-        for (int i = 0; i < VW; ++i) acc.x[i] = __shfl_sync(~0u, out.x[i], (W - 1) * L + lane % L);
-      }
+      if (cnt > 0) lastcd = scd[cnt - 1];
       __syncwarp();
-      if ((Mc >> (cnt - 1)) & 1u) touched &= ~(1u << top);
-      else touched |= 1u << top;
-      if (F >= 1 && M != 0u) {
-        if (lane == S - 1) nodeL += (uint32_t)__popc(M);
-        part &= ~(1u << (S - 1));
-      }
-      if (F >= 2 && M2 != 0u) {
-        if (lane == S - 2) nodeL += (uint32_t)__popc(M2);
-        part &= ~(1u << (S - 2));
-      }
-      int n = __popc(Mc);
-      uint32_t icd = compact_bits(Mc, cd - (uint32_t)(F + 1), xbuf, lane);
-      // the level loop: items of level l (node sums that closed in this batch)
-      for (int l = top; l >= d && n > 0; --l) {
-        const uint32_t first = __shfl_sync(~0u, nodeL, l);
-        const bool pfirst = (part >> l) & 1u;
-        const uint32_t fid =
-            (lane < n && (uint64_t)first + lane < a.nfibs[l]) ? __ldg(a.fids[l] + first + lane) : 0u;
-        float *store = a.store[l];
-        if (store != nullptr && (uint64_t)first + n <= a.nfibs[l]) {
-          float *sp = store + (size_t)first * a.ldr + col;
-          if (!pfirst) st_rows<V>(sp, 0, 0, 0, items[lane], act);
-          else if (a.span) st_rows<V>(span_row(a, chunk_id, l, 0), 0, 0, col, items[lane], act);
-          else red_rows<V>(sp, 0, 0, 0, items[lane], act);
-          for (int i = 1; i < n; ++i) {
-            sp += a.ldr;
-            st_rows<V>(sp, 0, 0, 0, items[i * 32 + lane], act);
-          }
-        }
-        if (l > d) {
-          const uint32_t Mp = __ballot_sync(~0u, lane < n && icd >= 1u);
-          const RowSrc<V, FT> Ul(a.U[l], a.ldr, col, act);
-          fv<V> cl = carry[(l - 1) * 32 + lane];
-          int jj = 0;
-  #pragma unroll 8
-          for (int i = 0; i < n; ++i) {
-            const fv<V> row = Ul.load(__shfl_sync(~0u, fid, i), true);
-            fv_fma(cl, items[i * 32 + lane], row);
-            if ((Mp >> i) & 1u) {
-              items[jj * 32 + lane] = cl;
-              cl = fv_fill<V>(0.f);
-              ++jj;
-            }
-          }
-          carry[(l - 1) * 32 + lane] = cl;
-          if ((Mp >> (n - 1)) & 1u) touched &= ~(1u << (l - 1));
-          else touched |= 1u << (l - 1);
-          if (lane == l) nodeL += (uint32_t)n;
-          part &= ~(1u << l);
-          icd = compact_bits(Mp, icd - 1u, xbuf, lane);
-          n = __popc(Mp);
-        } else {
-          for (int i = 0; i < n; ++i) {
-            const fv<V> val = items[i * 32 + lane];
-            const uint32_t orow = __shfl_sync(~0u, fid, i);
-            if (a.out == nullptr) {
-              // deterministic d > 0: the level-d sums went to a store row
-            } else if (d == 0) {
-              if (!(i == 0 && pfirst)) st_out<V>(a.out, orow, a.ldr, col, val, act);
-              else if (a.span) st_rows<V>(span_row(a, chunk_id, 0, 0), 0, 0, col, val, act);
-              else red_out<V>(a.out, orow, a.ldr, col, val, act);
-            } else {
-              red_out<V>(a.out, orow, a.ldr, col, fv_mul(val, pre[(d - 1) * 32 + lane]), act);
-              const uint32_t ci = __shfl_sync(~0u, icd, i);
-              if (ci >= 1u) nodeL = advance_prefix<V, FT>(a, pre, nodeL, d - (int)ci, d, col, act, lane);
-            }
-          }
-          if (lane == l) nodeL += (uint32_t)n;
-          part &= ~(1u << l);
-          n = 0;
-        }
-      }
     }
-    // chunk end: the open nodes of levels top .. d add their partial sums
-    // (the carried row, in the walker layout, is written by walker 0)
-    if (wk == 0)
-      *reinterpret_cast<fv<VW> *>(reinterpret_cast<float *>(carry) + (size_t)top * 32 * V + wcol) = acc;
-    __syncwarp();
-    for (int l = top; l >= d; --l) {
-      if (!((touched >> l) & 1u)) continue;
-      const uint32_t node = __shfl_sync(~0u, nodeL, l);
-      if ((uint64_t)node >= a.nfibs[l]) continue;
-      const fv<V> val = carry[l * 32 + lane];
-      if (a.store[l] != nullptr) {
-        if (a.span) st_rows<V>(span_row(a, chunk_id, l, 1), 0, 0, col, val, act);
-        else red_rows<V>(a.store[l], node, a.ldr, col, val, act);
-      }
-      if (l > d) {
-        const fv<V> r = ld_factor<V, FT>(a.U[l], __ldg(a.fids[l] + node), a.ldr, col, act);
-        fv<V> c2 = carry[(l - 1) * 32 + lane];
-        fv_fma(c2, val, r);
-        carry[(l - 1) * 32 + lane] = c2;
-        touched |= 1u << (l - 1);
-      } else if (a.out != nullptr) {
-        if (a.span && d == 0) {
-          st_rows<V>(span_row(a, chunk_id, 0, 1), 0, 0, col, val, act);
-        } else {
-          const uint32_t orow = __ldg(a.fids[d] + node);
-          red_out<V>(a.out, orow, a.ldr, col, d == 0 ? val : fv_mul(val, pre[(d - 1) * 32 + lane]),
-                     act);
+    // chunk end: the nodes that the last unit did not close go on in the next
+    // chunk; their partial sums go to the tail rows, or into their parents'
+    if (live) {
+      Row<VW> x = acc;  // what the level holds, with what the level below adds
+      for (int l = top; l >= d; --l) {
+        if (l < top) x = row_add(x, carry[l * 32]);
+        if (l < S - (int)lastcd) {
+          const uint32_t n = l == top ? nt : nodes[l * 32];
+          if (a.span_lev[l] >= 0 && act) *reinterpret_cast<Row<VW> *>(span_row(a, chunk_id, l, 1) + col) = x;
+          if (l > d)
+            x = row_mul(x, ld_row<VW, FT>(row_at(static_cast<const char *>(a.U[l]),
+                                                 __ldg(a.fids[l] + n), stride) + lane_off));
         }
       }
     }
     __syncwarp();
-    chunk_id = claims ? __shfl_sync(~0u, claim, 0) : a.nchunks;
+    group = a.counter != nullptr ? gridDim.x * kWarps + __shfl_sync(~0u, claim, 0) : ngroups;
   }
 }
 
@@ -1139,6 +1207,7 @@ WalkArgs make_args(const TreeWalk &w, const LevelFactors *f, double *out) {
   a.nunits = w.nunits;
   for (int l = 0; l < kMaxModes; ++l) {
     a.nfibs[l] = c.nfibs[l];
+    a.dims[l] = l < c.nmodes ? c.dims[c.dim_perm[l]] : 0;
     a.fptr[l] = c.fptr[l].get();
     a.fids[l] = c.fids[l].get();
     a.U[l] = f ? f->U[l] : nullptr;
@@ -1148,7 +1217,6 @@ WalkArgs make_args(const TreeWalk &w, const LevelFactors *f, double *out) {
   a.src_rows = w.src_rows;
   a.src_ids = c.fids[w.src].get();
   a.src_cd = w.src >= 1 ? c.cdepth[w.src].get() : nullptr;
-  a.U_src = f ? f->U[w.src] : nullptr;
   a.out = out;
   a.sched = w.sched.get();
   a.counter = w.sched.get() ? w.sched.get() + (size_t)w.nchunks * (w.src + 1) : nullptr;
@@ -1171,41 +1239,84 @@ unsigned resident_blocks(K kernel, int threads, size_t smem) {
   return (unsigned)std::max(1, sms * std::max(1, per_sm));
 }
 
-template <int V, int W, int VW, FactorType FT, bool LEAF, int F>
-void launch_contract_v(const WalkArgs &a, unsigned blocks, bool resident, cudaStream_t s) {
-  const size_t smem = contract_smem<V>(a.N);
-  auto kern = k_contract<V, W, VW, FT, LEAF, F>;
-  if (resident) {
-    blocks = std::min(blocks, resident_blocks(kern, 256, smem));
-    ADATM_CUDA(cudaMemsetAsync(a.counter, 0, sizeof(uint32_t), s));
-    kern<<<blocks, 256, smem, s>>>(a);
-  } else {
-    WalkArgs b = a;
-    b.counter = nullptr;  // one chunk per warp: blocks cover every chunk
-    kern<<<blocks, 256, smem, s>>>(b);
-  }
+// The lowest factor of the source level and the f levels above it.
+const void *hot_base(const WalkArgs &a, int f) {
+  const char *b = static_cast<const char *>(a.U[a.S]);
+  for (int i = 0; i < f; ++i) b = std::min(b, static_cast<const char *>(a.U[a.S - 1 - i]));
+  return b;
 }
 
-// Levels folded into the source loop: level S-1 whenever it is neither
-// stored nor the output level (a level-(S-1) item costs more than the extra
-// gather per unit at any fan-out the trees show); level S-2 as well when it
-// too is unstored and above d and holds at most kFold2Units source units per
-// node on average (at higher fan-out the extra gather per unit costs more
-// than the items it saves). `want` >= 0 caps the count.
-constexpr double kFold2Units = 4.0;
-int fold_levels(const WalkArgs &a, int want) {
-  const int cap = want < 0 ? 2 : std::min(want, 2);
+template <int W, int VW, FactorType FT, bool LEAF, int F>
+void launch_contract_v(const WalkArgs &a, bool resident, cudaStream_t s) {
+  const size_t smem = kWarps * contract_warp_smem<W, VW, F>(a.d, a.S - 1 - F);
+  auto kern = k_contract<W, VW, FT, LEAF, F>;
+  const unsigned groups = (a.nchunks + W - 1) / W;
+  unsigned blocks = (groups + kWarps - 1) / kWarps;
+  WalkArgs b = a;
+  const int top = a.S - 1 - F;
+  HotArgs h = {};
+  h.base = hot_base(a, F);
+  const size_t stride = (size_t)a.ldr * (FT == FactorType::F32 ? 4 : 2);
+  auto first_row = [&](int l) {
+    return (uint32_t)((static_cast<const char *>(a.U[l]) - static_cast<const char *>(h.base)) / stride);
+  };
+  h.src_row = first_row(a.S);
+  for (int f = 0; f < F; ++f) {
+    h.fold_row[f] = first_row(a.S - 1 - f);
+    h.fold_ids[f] = a.fids[a.S - 1 - f];
+  }
+  h.top_ids = a.fids[top];
+  h.top_rows = a.U[top];
+  h.top_last = (uint32_t)a.nfibs[top] - 1u;
+  h.top_store = a.store[top];
+  h.top_keep = a.span_lev[top] >= 0;
+  if (resident) blocks = std::min(blocks, resident_blocks(kern, 256, smem));
+  if (blocks * kWarps < groups) ADATM_CUDA(cudaMemsetAsync(b.counter, 0, sizeof(uint32_t), s));
+  else b.counter = nullptr;  // a group of chunks for every warp: nothing to claim
+  kern<<<blocks, 256, smem, s>>>(b, h);
+}
+
+// Levels folded into the source loop, from level S-1 up: levels that are
+// neither stored nor the output, as long as they hold at most fold_units()
+// source units per node on average: at higher fan-out the extra row per unit
+// costs more than the closes it saves. `want` >= 0 caps the count.
+//
+// Measured (ms per MTTKRP, fold up to 4 / 10 / 30 units per node): FP32, R =
+// 32, the 6th-order tensor's second and third contractions 2.18 / 2.26 / 2.26
+// and 1.97 / 1.97 / 2.16; BF16 rows (half the L1 bytes per row), R = 64, the
+// 5th-order tensor's second contraction 1.44 / 1.25 / 1.25.
+template <FactorType FT>
+constexpr double fold_units() {
+  return FT == FactorType::F32 ? 5.0 : 10.0;
+}
+int fold_levels(const WalkArgs &a, int want, double units, size_t stride) {
+  const int cap = want < 0 ? kMaxFold : std::min(want, kMaxFold);
   int f = 0;
-  while (f < cap && a.S - 1 - f > a.d && a.store[a.S - 1 - f] == nullptr) ++f;
-  if (want < 0 && f == 2 && (double)a.nunits > kFold2Units * (double)a.nfibs[a.S - 2]) f = 1;
+  while (f < cap && a.S - 1 - f > a.d && a.store[a.S - 1 - f] == nullptr &&
+         (want >= 0 || f == 0 || (double)a.nunits <= units * (double)a.nfibs[a.S - 1 - f]))
+    ++f;
+  // the unit loop addresses the rows of its levels from the lowest factor on,
+  // in 32-bit units of four columns (a single factor that fits the device does)
+  const uint64_t unit = stride / (uint64_t)(a.ldr / 4);
+  auto numbered = [&](int n) {
+    const char *b = static_cast<const char *>(hot_base(a, n));
+    for (int l = a.S; l >= a.S - n; --l) {
+      const uint64_t off = (uint64_t)(static_cast<const char *>(a.U[l]) - b);
+      if (off % stride != 0 || off / unit + a.dims[l] * (uint64_t)(a.ldr / 4) > 0xFFFFFFFFull) return false;
+    }
+    return true;
+  };
+  while (f > 0 && !numbered(f)) --f;
   return f;
 }
 
-// The (V, W, VW) shapes the contraction is built for: V columns per lane in
-// the level loop (32 lanes cover the rank), W walkers in the source loop
-// with VW columns per lane (32 / W lanes cover the rank).
+// The (W, VW) shapes the contraction is built for: W walkers per warp with VW
+// columns per lane (32 / W lanes cover the rank).
 #define ADATM_CONTRACT_SHAPES(X) \
-  X(1, 1, 1) X(1, 2, 1) X(1, 2, 2) X(1, 4, 1) X(1, 4, 2) X(1, 4, 4) X(2, 1, 2) X(2, 2, 4) X(4, 1, 4)
+  X(1, 1) X(1, 2) X(1, 4) X(2, 1) X(2, 2) X(2, 4) X(4, 1) X(4, 2) X(4, 4) X(8, 1) X(8, 2) X(8, 4)
+// Folded levels beyond the second are built for the default shapes above rank
+// 8 (four columns per lane).
+constexpr int max_fold(int vw) { return vw == 4 ? kMaxFold : 2; }
 
 // Columns per walker lane for W walkers at rank R (0 if W walkers cannot
 // cover R with at most 4 columns per lane).
@@ -1216,17 +1327,22 @@ int walker_cols(int R, int W) {
 }
 
 template <FactorType FT, bool LEAF>
-void launch_contract(int vec, int walkers, int fold, const WalkArgs &a, unsigned blocks, bool resident,
-                     cudaStream_t s) {
-  const int f = fold_levels(a, fold);
+void launch_contract(int walkers, int fold, const WalkArgs &a, bool resident, cudaStream_t s) {
   const int vw = walker_cols(a.R, walkers);
-#define ADATM_CONTRACT_CASE(V, W, VW)                                                  \
-  if (vec == V && walkers == W && vw == VW) {                                          \
-    if (f == 2) launch_contract_v<V, W, VW, FT, LEAF, 2>(a, blocks, resident, s);      \
-    else if (f == 1) launch_contract_v<V, W, VW, FT, LEAF, 1>(a, blocks, resident, s); \
-    else launch_contract_v<V, W, VW, FT, LEAF, 0>(a, blocks, resident, s);             \
-    ADATM_LAUNCH();                                                                    \
-    return;                                                                            \
+  const int f = std::min(
+      fold_levels(a, fold, fold_units<FT>(), (size_t)a.ldr * (FT == FactorType::F32 ? 4 : 2)), max_fold(vw));
+#define ADATM_CONTRACT_CASE(W, VW)                                                      \
+  if (walkers == W && vw == VW) {                                                       \
+    if constexpr (max_fold(VW) > 2) {                                                   \
+      if (f == 5) launch_contract_v<W, VW, FT, LEAF, 5>(a, resident, s);                \
+      else if (f == 4) launch_contract_v<W, VW, FT, LEAF, 4>(a, resident, s);           \
+      else if (f == 3) launch_contract_v<W, VW, FT, LEAF, 3>(a, resident, s);           \
+    }                                                                                   \
+    if (f == 2) launch_contract_v<W, VW, FT, LEAF, 2>(a, resident, s);                  \
+    else if (f == 1) launch_contract_v<W, VW, FT, LEAF, 1>(a, resident, s);             \
+    else if (f == 0) launch_contract_v<W, VW, FT, LEAF, 0>(a, resident, s);             \
+    ADATM_LAUNCH();                                                                     \
+    return;                                                                             \
   }
   ADATM_CONTRACT_SHAPES(ADATM_CONTRACT_CASE)
 #undef ADATM_CONTRACT_CASE
@@ -1268,18 +1384,11 @@ int vec_for_rank(int R) {
 
 }  // namespace
 
-int default_walkers(int R) { return R <= 64 ? 2 : 1; }
+// As many walkers as cover the rank at four columns (one 16-byte load) per lane.
+int default_walkers(int R) { return R <= 16 ? 8 : (R <= 32 ? 4 : (R <= 64 ? 2 : 1)); }
 
 bool walkers_supported(int R, int W) {
-  if (W != 1 && W != 2 && W != 4) return false;
-  const int v = R <= 32 ? 1 : (R <= 64 ? 2 : 4);
-  const int vw = walker_cols(R, W);
-  if (vw == 0) return false;
-#define ADATM_CONTRACT_OK(V, WW, VW) \
-  if (v == V && W == WW && vw == VW) return true;
-  ADATM_CONTRACT_SHAPES(ADATM_CONTRACT_OK)
-#undef ADATM_CONTRACT_OK
-  return false;
+  return (W == 1 || W == 2 || W == 4) && R <= 128 && walker_cols(R, W) != 0;
 }
 
 namespace {
@@ -1298,19 +1407,24 @@ int lanes_for_rank(int R) {
 void set_walk_attributes() {
   static bool done = false;
   if (done) return;
-#define ADATM_ATTR_C0(V, W, VW, FT, LEAF, F)                                      \
-  ADATM_CUDA(cudaFuncSetAttribute(k_contract<V, W, VW, FT, LEAF, F>,              \
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize,    \
-                                  (int)contract_smem<V>(kMaxModes)));
-#define ADATM_ATTR_C1(V, W, VW, FT, LEAF) \
-  ADATM_ATTR_C0(V, W, VW, FT, LEAF, 0)    \
-  ADATM_ATTR_C0(V, W, VW, FT, LEAF, 1)    \
-  ADATM_ATTR_C0(V, W, VW, FT, LEAF, 2)
-#define ADATM_ATTR_CS(V, W, VW)                       \
-  ADATM_ATTR_C1(V, W, VW, FactorType::F32, true)      \
-  ADATM_ATTR_C1(V, W, VW, FactorType::F32, false)     \
-  ADATM_ATTR_C1(V, W, VW, FactorType::BF16, true)     \
-  ADATM_ATTR_C1(V, W, VW, FactorType::BF16, false)
+#define ADATM_ATTR_C0(W, VW, FT, LEAF, F)                                       \
+  ADATM_CUDA(cudaFuncSetAttribute(k_contract<W, VW, FT, LEAF, F>,               \
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize,  \
+                                  (int)(kWarps * contract_warp_smem<W, VW, F>(0, kMaxModes - 2 - F))));
+#define ADATM_ATTR_C1(W, VW, FT, LEAF)       \
+  ADATM_ATTR_C0(W, VW, FT, LEAF, 0)          \
+  ADATM_ATTR_C0(W, VW, FT, LEAF, 1)          \
+  ADATM_ATTR_C0(W, VW, FT, LEAF, 2)          \
+  if constexpr (max_fold(VW) > 2) {          \
+    ADATM_ATTR_C0(W, VW, FT, LEAF, 3)        \
+    ADATM_ATTR_C0(W, VW, FT, LEAF, 4)        \
+    ADATM_ATTR_C0(W, VW, FT, LEAF, 5)        \
+  }
+#define ADATM_ATTR_CS(W, VW)                       \
+  ADATM_ATTR_C1(W, VW, FactorType::F32, true)      \
+  ADATM_ATTR_C1(W, VW, FactorType::F32, false)     \
+  ADATM_ATTR_C1(W, VW, FactorType::BF16, true)     \
+  ADATM_ATTR_C1(W, VW, FactorType::BF16, false)
 #define ADATM_ATTR_S(W, FT, LEAF)                                                 \
   ADATM_CUDA(cudaFuncSetAttribute(k_scatter<W, FT, LEAF, false>,                  \
                                   cudaFuncAttributeMaxDynamicSharedMemorySize,    \
@@ -1358,19 +1472,32 @@ void to_device(DevBuf<T> &dst, const std::vector<T> &h, cudaStream_t s) {
   ADATM_CUDA(cudaStreamSynchronize(s));
 }
 
-// Slots and chains of a contraction: levels whose cut nodes would otherwise
-// take atomics (stored levels, and level 0 when it is the output), and for
-// each node a chunk boundary cuts, the run of chunks it spans. Deterministic
-// contractions below the root also store their level-d sums for the pull.
+// Slots and chains of a contraction: the levels whose cut nodes are summed
+// over chunks (stored levels, and level 0 when it is the output), and for
+// each node a chunk boundary cuts, the run of chunks it spans. Contractions
+// below the root also store their level-d sums for the pull or the scatter.
 void prepare_spans(TreeWalk &w, cudaStream_t s) {
   const DevCsf &c = *w.csf;
   const int S = w.src, d = w.out;
-  if (w.deterministic && d > 0) {
-    // the level-d sums are stored, then pulled into the output rows
+  if (d > 0) {
+    // the level-d sums are stored, then pulled (or, with atomics, scattered)
+    // into the output rows
     w.level_rows.alloc((size_t)std::max<uint64_t>(c.nfibs[d], 1) * w.ldr);
     ADATM_CUDA(cudaMemsetAsync(w.level_rows.get(), 0, w.level_rows.bytes(), s));
     w.store[d] = w.level_rows.get();
-    w.pull = true;
+    if (w.deterministic) {
+      w.pull = true;
+    } else {
+      w.scatter = std::make_unique<TreeWalk>();
+      TreeWalk &t = *w.scatter;
+      t.csf = w.csf;
+      t.R = w.R;
+      t.ldr = w.ldr;
+      t.src = t.out = d;
+      t.src_rows = w.level_rows.get();
+      t.chunk = kScatterChunk;
+      walk_prepare(t, s);
+    }
   }
   w.span_nlev = 0;
   for (int l = 0; l < kMaxModes; ++l) w.span_lev[l] = -1;
@@ -1634,12 +1761,32 @@ void find_hot_rows(TreeWalk &w, cudaStream_t s) {
   w.nhot = (int)hot.size();
 }
 
+// Source units per chunk where the caller names none. A scatter's chunk is a
+// warp's; a contraction's is a walker's, and every walker slot of a resident
+// grid (4 blocks of 8 warps per SM) should have work: one chunk per slot while
+// that is at most kMaxChunk units (all slots then run once, side by side),
+// else chunks small enough that the last ones leave few slots idle.
+//
+// Measured (us per MTTKRP sequence, chunks of 16 / 32 / 64 / 128): 1M units,
+// R = 16 (26 units per slot) 154 / 145 / 154 / 187; 1.9M units, R = 24 (90
+// per slot) 451 / 404 / 391 / 373; 3.5M units, R = 32 (185 per slot) 955 /
+// 874 / 869 / 939; 55K units, R = 16 140 / 165 / 215 / -.
+uint32_t auto_chunk(const TreeWalk &w) {
+  if (w.src == w.out) return w.src == w.nmodes - 1 ? 2 * kScatterChunk : kScatterChunk;
+  constexpr uint64_t kMaxChunk = 128, kMinChunk = 16;
+  const uint64_t slots = 148ull * 32 * default_walkers(w.R);
+  const uint64_t per_slot = (w.nunits + slots - 1) / slots;
+  const uint64_t c = per_slot <= kMaxChunk ? per_slot : std::min(kMaxChunk, per_slot / 4);
+  return (uint32_t)std::max(kMinChunk, (c + 15) / 16 * 16);
+}
+
 void walk_prepare(TreeWalk &w, cudaStream_t s) {
   set_walk_attributes();
   const DevCsf &c = *w.csf;
   w.nmodes = c.nmodes;
   w.nunits = c.nfibs[w.src];
-  if (w.chunk == 0) w.chunk = 32;
+  if (w.chunk == 0) w.chunk = auto_chunk(w);
+  w.chunk = std::min(w.chunk, 1u << 30);  // offsets in a chunk are 32-bit numbers
   w.nchunks = (uint32_t)((w.nunits + w.chunk - 1) / w.chunk);
   w.sched.alloc((size_t)std::max<uint32_t>(w.nchunks, 1) * (w.src + 1) + 1);  // + the chunk counter
   w.nhot = 0;
@@ -1662,22 +1809,22 @@ void walk_launch(const TreeWalk &w, const LevelFactors &f, FactorType ft, double
     launch_pull(w, f, ft, w.src == w.nmodes - 1 ? nullptr : w.src_rows, out, s);
     return;
   }
-  const WalkArgs a = make_args(w, &f, w.deterministic && w.out > 0 ? nullptr : out);
-  const unsigned blocks = (unsigned)((w.nchunks + kWarps - 1) / kWarps);
+  const WalkArgs a = make_args(w, &f, w.src > w.out && w.out > 0 ? nullptr : out);
   const bool leaf = w.src == w.nmodes - 1;
   if (w.src > w.out) {
-    const int vec = vec_for_rank(w.R);
     const int wk = w.walkers > 0 ? w.walkers : default_walkers(w.R);
     if (ft == FactorType::F32) {
-      if (leaf) launch_contract<FactorType::F32, true>(vec, wk, w.fold, a, blocks, w.resident, s);
-      else launch_contract<FactorType::F32, false>(vec, wk, w.fold, a, blocks, w.resident, s);
+      if (leaf) launch_contract<FactorType::F32, true>(wk, w.fold, a, w.resident, s);
+      else launch_contract<FactorType::F32, false>(wk, w.fold, a, w.resident, s);
     } else {
-      if (leaf) launch_contract<FactorType::BF16, true>(vec, wk, w.fold, a, blocks, w.resident, s);
-      else launch_contract<FactorType::BF16, false>(vec, wk, w.fold, a, blocks, w.resident, s);
+      if (leaf) launch_contract<FactorType::BF16, true>(wk, w.fold, a, w.resident, s);
+      else launch_contract<FactorType::BF16, false>(wk, w.fold, a, w.resident, s);
     }
     launch_chains(w, out, s);
-    if (w.deterministic && w.out > 0) launch_pull(w, f, ft, w.level_rows.get(), out, s);
+    if (w.scatter) walk_launch(*w.scatter, f, ft, out, s);
+    else if (w.out > 0) launch_pull(w, f, ft, w.level_rows.get(), out, s);
   } else {
+    const unsigned blocks = (unsigned)((w.nchunks + kWarps - 1) / kWarps);
     const int lanes = lanes_for_rank(w.R);
     if (ft == FactorType::F32) {
       if (leaf) launch_scatter<FactorType::F32, true>(lanes, a, blocks, s);
@@ -1698,6 +1845,7 @@ int walk_kernels(const TreeWalk &w) {
   }
   if (w.deterministic && w.nsegs) k += w.out + 1 + (w.nlong ? 1 : 0);  // prefix levels, pull, pieces
   if (!w.deterministic && w.src == w.out) k += 1;      // the scatter
+  if (w.scatter) k += walk_kernels(*w.scatter);
   return k;
 }
 

@@ -8,20 +8,21 @@
 //    stored memo row T_S) is multiplied by its factor row and summed into its
 //    level S-1 parent; a completed node of level l > d multiplies its sum by
 //    its own factor row and adds it to its parent; a completed node of level
-//    d is written to the output row fids[d][node], multiplied by the prefix
-//    product P_{d-1} of the factor rows on its root path (d > 0). Completed
-//    nodes of the levels listed in `store` are also written to memo rows.
+//    d is written to the output row fids[d][node] (d = 0), or to a row of its
+//    own that is then pulled or scattered like a memo row. Completed nodes of
+//    the levels listed in `store` are also written to memo rows.
 //  * scatter (S == d): every unit u adds src(u) * P_{d-1} to output row
-//    fids[d][u] (leaf MTTKRP when d = N-1, memo reuse at its stored level).
+//    fids[d][u], P_{d-1} the product of the factor rows on the root path of
+//    its parent (leaf MTTKRP when d = N-1, memo reuse at its stored level).
 //
 // Work is split into chunks of `chunk` consecutive source units, one chunk
-// per row group of LANES lanes (each lane holds 4 of the R columns), so the
-// split follows nonzeros, not root slices (the reference's omp
-// schedule(dynamic,16) over slices, mttkrp.c:392, cannot balance a slice
-// holding 16% of the nonzeros). Nodes cut by a chunk boundary are combined
-// with vector atomics; for memo rows those nodes are zeroed first by a
-// separate launch, all other memo rows are written exactly once.
+// per walker (a group of lanes), so the split follows nonzeros, not root
+// slices (the reference's omp schedule(dynamic,16) over slices,
+// mttkrp.c:392, cannot balance a slice holding 16% of the nonzeros). The
+// partial sums of nodes cut by a chunk boundary are added in chunk order.
 #pragma once
+
+#include <memory>
 
 #include "csf_build.cuh"
 
@@ -40,7 +41,7 @@ struct TreeWalk {
   int src = 0;                 // source level S
   int out = 0;                 // output level d
   int R = 0, ldr = 0;
-  uint32_t chunk = 32;
+  uint32_t chunk = 0;          // source units per chunk (0 = by size, walk_prepare)
   uint32_t nchunks = 0;
   uint64_t nunits = 0;         // nodes of level S
   const DevCsf *csf = nullptr;
@@ -48,12 +49,12 @@ struct TreeWalk {
   float *store[kMaxModes] = {nullptr};       // memo rows written, per level
   DevBuf<uint32_t> sched;                    // nchunks x (S + 1), then the chunk counter
   bool resident = true;                      // contraction grid: resident blocks that claim
-                                             // chunks (else one chunk per warp)
-  int walkers = 0;                           // contraction source loop: walkers per warp
-                                             // (1, 2 or 4; 0 = default_walkers(R))
-  int fold = -1;                             // contraction: unstored levels below the
+                                             // chunks (else a group of chunks per warp)
+  int walkers = 0;                           // contraction: walkers per warp (1, 2 or 4;
+                                             // 0 = default_walkers(R))
+  int fold = -1;                             // contraction: unstored levels above the
                                              // source folded into its loop (0..2; -1 =
-                                             // chosen from the tree's fan-out)
+                                             // as many as the tree's fan-out suggests)
   // Scatter walks: the output rows that the most units hit (at most
   // kHotRows, each hit by at least kHotMin units) are summed per block in
   // shared memory; hot_slot maps an output row to its slot (0xFF = none).
@@ -81,6 +82,7 @@ struct TreeWalk {
   DevBuf<uint32_t> chain_ids;        // chains of few groups first (nshort), then long ones
   uint32_t nshort = 0;
   DevBuf<float> level_rows;          // contraction below the root: level-d node sums
+  std::unique_ptr<TreeWalk> scatter; // and, with atomics, their scatter into the output rows
   // pull scatter of level `out` (deterministic scatters and contractions below the root)
   bool pull = false;
   DevBuf<uint32_t> parent[kMaxModes];  // parent node of every node of levels 1..out
@@ -100,8 +102,8 @@ struct TreeWalk {
 // Kernel launches of one walk (for launch counts).
 int walk_kernels(const TreeWalk &w);
 
-// Walkers per warp of the contraction's source loop by default at rank R,
-// and whether W walkers are built for rank R.
+// Walkers per warp of a contraction by default at rank R, and whether a
+// caller may choose W walkers at rank R.
 int default_walkers(int R);
 bool walkers_supported(int R, int W);
 

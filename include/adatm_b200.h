@@ -230,7 +230,7 @@ int adatm_plan_splatt(const adatm_tensor *t, int csf_alloc, adatm_plan *out);
 /* Engine: trees, memo rows and factors for one plan and rank.
  * factor_bf16 != 0 keeps a BF16 copy of every factor for the gathers
  * (accumulation stays FP32). chunk_leaf/chunk_rows: source units per chunk
- * (0 = defaults). The engine copies what it needs from the tensor. */
+ * (0 = chosen from the number of units). The engine copies what it needs from the tensor. */
 int adatm_engine_create(const adatm_tensor *t, uint64_t rank, const adatm_plan *plan,
                         int factor_bf16, uint32_t chunk_leaf, uint32_t chunk_rows,
                         adatm_engine **out);
@@ -308,8 +308,8 @@ int adatm_engine_autotune(adatm_engine *e, const uint32_t *chunk_leaf, const uin
  * Drops a captured sweep. No reference counterpart (a launch-shape control). */
 int adatm_engine_set_resident_grid(adatm_engine *e, int on);
 
-/* Walkers per warp in the contraction walks' source loop: 1, 2 or 4 (0 =
- * the default for the rank). With W walkers one warp instruction advances W
+/* Walkers per warp in the contraction walks: 1, 2 or 4 (0 = the default for
+ * the rank). With W walkers one warp instruction advances W
  * source units (32/W lanes and up to 4 columns per lane each); refused with
  * SPLATT_ERROR_BADINPUT where W walkers cannot cover the rank. Results agree
  * up to FP32 summation order. Drops a captured sweep. No reference
@@ -317,8 +317,8 @@ int adatm_engine_set_resident_grid(adatm_engine *e, int on);
 int adatm_engine_set_walkers(adatm_engine *e, int walkers);
 
 /* Unstored tree levels folded into the contraction walks' source loop: 0, 1
- * or 2 (-1, the default: level S-1 whenever it can be, level S-2 too where
- * its nodes hold at most 4 source units on average). A folded level's nodes
+ * or 2 (-1, the default: level S-1 whenever it can be, and the levels above
+ * it, five at most, where their nodes hold few source units on average). A folded level's nodes
  * are not formed: each source unit is multiplied by its ancestors' factor
  * rows directly. Refused with SPLATT_ERROR_BADINPUT outside -1..2. Results
  * agree up to FP32 summation order. Drops a captured sweep. No reference
