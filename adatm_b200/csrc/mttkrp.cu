@@ -3,7 +3,7 @@
 #include <type_traits>
 #include <vector>
 
-#include "mttkrp.cuh"
+#include "rows.cuh"
 
 namespace adatm {
 
@@ -51,357 +51,6 @@ constexpr uint64_t kHotScanRows = 1ull << 24;  // output rows the hot-row search
 constexpr int kWarps = 8;   // warps per block
 constexpr int kBatch = 32;  // units per batch of a scatter or pull warp
 
-template <int V>
-struct alignas(sizeof(float) * V) fv {
-  float x[V];
-};
-
-template <int V>
-__device__ __forceinline__ fv<V> fv_fill(float s) {
-  fv<V> r;
-#pragma unroll
-  for (int i = 0; i < V; ++i) r.x[i] = s;
-  return r;
-}
-// Pairs of columns go through the packed FP32 instructions (one issue slot
-// for two products; each is rounded as its scalar form is).
-__device__ __forceinline__ uint64_t pack2(float x, float y) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
-  return r;
-}
-__device__ __forceinline__ void unpack2(uint64_t p, float &x, float &y) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(p));
-}
-template <int V>
-__device__ __forceinline__ fv<V> fv_mul(const fv<V> &a, const fv<V> &b) {
-  fv<V> r;
-  if constexpr (V == 1) {
-    r.x[0] = a.x[0] * b.x[0];
-  } else {
-#pragma unroll
-    for (int i = 0; i < V; i += 2) {
-      uint64_t t;
-      asm("mul.rn.f32x2 %0, %1, %2;"
-          : "=l"(t)
-          : "l"(pack2(a.x[i], a.x[i + 1])), "l"(pack2(b.x[i], b.x[i + 1])));
-      unpack2(t, r.x[i], r.x[i + 1]);
-    }
-  }
-  return r;
-}
-
-// Columns col..col+V-1 of factor row `row` (FP32 or BF16 storage).
-template <int V, FactorType FT>
-__device__ __forceinline__ fv<V> ld_factor(const void *U, uint32_t row, int ldr, int col, bool act) {
-  fv<V> r = fv_fill<V>(0.f);
-  if (!act) return r;
-  if constexpr (FT == FactorType::F32) {
-    const float *p = static_cast<const float *>(U) + (size_t)row * ldr + col;
-    if constexpr (V == 1) {
-      r.x[0] = __ldg(p);
-    } else if constexpr (V == 2) {
-      const float2 t = __ldg(reinterpret_cast<const float2 *>(p));
-      r.x[0] = t.x;
-      r.x[1] = t.y;
-    } else {
-      const float4 t = __ldg(reinterpret_cast<const float4 *>(p));
-      r.x[0] = t.x;
-      r.x[1] = t.y;
-      r.x[2] = t.z;
-      r.x[3] = t.w;
-    }
-  } else {
-    const __nv_bfloat16 *p = static_cast<const __nv_bfloat16 *>(U) + (size_t)row * ldr + col;
-    if constexpr (V == 1) {
-      r.x[0] = __bfloat162float(__ldg(p));
-    } else if constexpr (V == 2) {
-      const float2 t = __bfloat1622float2(__ldg(reinterpret_cast<const __nv_bfloat162 *>(p)));
-      r.x[0] = t.x;
-      r.x[1] = t.y;
-    } else {
-      const uint2 raw = __ldg(reinterpret_cast<const uint2 *>(p));
-      const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&raw.x));
-      const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&raw.y));
-      r.x[0] = lo.x;
-      r.x[1] = lo.y;
-      r.x[2] = hi.x;
-      r.x[3] = hi.y;
-    }
-  }
-  return r;
-}
-
-// FP32 row matrices (memo rows, outputs).
-template <int V>
-__device__ __forceinline__ fv<V> ld_rows(const float *base, uint64_t row, int ldr, int col, bool act) {
-  fv<V> r = fv_fill<V>(0.f);
-  if (!act) return r;
-  const float *p = base + row * (uint64_t)ldr + col;
-  if constexpr (V == 1) {
-    r.x[0] = __ldg(p);
-  } else if constexpr (V == 2) {
-    const float2 t = __ldg(reinterpret_cast<const float2 *>(p));
-    r.x[0] = t.x;
-    r.x[1] = t.y;
-  } else {
-    const float4 t = __ldg(reinterpret_cast<const float4 *>(p));
-    r.x[0] = t.x;
-    r.x[1] = t.y;
-    r.x[2] = t.z;
-    r.x[3] = t.w;
-  }
-  return r;
-}
-
-// FP64 output rows: the MTTKRP sums of a row can come from millions of
-// units (a skewed slice), and FP32 sums of that many partials lose several
-// digits; outputs are stored and added in FP64.
-template <int V>
-__device__ __forceinline__ void st_out(double *base, uint64_t row, int ldr, int col, const fv<V> &v,
-                                       bool act) {
-  if (!act) return;
-  double *p = base + row * (uint64_t)ldr + col;
-  if constexpr (V == 1) {
-    *p = v.x[0];
-  } else if constexpr (V == 2) {
-    *reinterpret_cast<double2 *>(p) = make_double2(v.x[0], v.x[1]);
-  } else {
-    *reinterpret_cast<double2 *>(p) = make_double2(v.x[0], v.x[1]);
-    *reinterpret_cast<double2 *>(p + 2) = make_double2(v.x[2], v.x[3]);
-  }
-}
-
-// Factor-row gathers through a per-lane base pointer (the lane's first
-// column) and a byte stride, so an address is one wide multiply-add.
-template <int V, FactorType FT>
-struct RowSrc {
-  const char *base = nullptr;
-  uint32_t stride = 0;
-  RowSrc() = default;
-  // Lanes past the rank read column 0 (their results are never stored).
-  __device__ __forceinline__ RowSrc(const void *U, int ldr, int col, bool act) {
-    constexpr int esz = FT == FactorType::F32 ? 4 : 2;
-    base = static_cast<const char *>(U) + (size_t)(act ? col : 0) * esz;
-    stride = (uint32_t)ldr * esz;
-  }
-  __device__ __forceinline__ fv<V> load(uint32_t row) const {
-    fv<V> r;
-    const char *p = base + (size_t)row * stride;
-    if constexpr (FT == FactorType::F32) {
-      if constexpr (V == 1) {
-        r.x[0] = __ldg(reinterpret_cast<const float *>(p));
-      } else if constexpr (V == 2) {
-        const float2 t = __ldg(reinterpret_cast<const float2 *>(p));
-        r.x[0] = t.x;
-        r.x[1] = t.y;
-      } else {
-        const float4 t = __ldg(reinterpret_cast<const float4 *>(p));
-        r.x[0] = t.x;
-        r.x[1] = t.y;
-        r.x[2] = t.z;
-        r.x[3] = t.w;
-      }
-    } else {
-      if constexpr (V == 1) {
-        r.x[0] = __bfloat162float(__ldg(reinterpret_cast<const __nv_bfloat16 *>(p)));
-      } else if constexpr (V == 2) {
-        const float2 t = __bfloat1622float2(__ldg(reinterpret_cast<const __nv_bfloat162 *>(p)));
-        r.x[0] = t.x;
-        r.x[1] = t.y;
-      } else {
-        const uint2 raw = __ldg(reinterpret_cast<const uint2 *>(p));
-        const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&raw.x));
-        const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&raw.y));
-        r.x[0] = lo.x;
-        r.x[1] = lo.y;
-        r.x[2] = hi.x;
-        r.x[3] = hi.y;
-      }
-    }
-    return r;
-  }
-};
-
-// V columns as packed pairs (one register pair for two FP32 columns), the
-// form the contraction keeps its rows in: no moves between loads and the
-// packed products.
-template <int V>
-struct alignas(4 * V) Row {
-  uint64_t w[V / 2];
-};
-template <>
-struct alignas(4) Row<1> {
-  float w;
-};
-template <int V>
-__device__ __forceinline__ Row<V> row_zero() {
-  Row<V> r;
-  if constexpr (V == 1) {
-    r.w = 0.f;
-  } else {
-#pragma unroll
-    for (int i = 0; i < V / 2; ++i) r.w[i] = 0ull;
-  }
-  return r;
-}
-template <int V>
-__device__ __forceinline__ fv<V> row_values(const Row<V> &r) {
-  fv<V> f;
-  if constexpr (V == 1) {
-    f.x[0] = r.w;
-  } else {
-#pragma unroll
-    for (int i = 0; i < V / 2; ++i) unpack2(r.w[i], f.x[2 * i], f.x[2 * i + 1]);
-  }
-  return f;
-}
-template <int V>
-__device__ __forceinline__ Row<V> row_mul(const Row<V> &a, const Row<V> &b) {
-  Row<V> r;
-  if constexpr (V == 1) {
-    r.w = a.w * b.w;
-  } else {
-#pragma unroll
-    for (int i = 0; i < V / 2; ++i)
-      asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.w[i]) : "l"(a.w[i]), "l"(b.w[i]));
-  }
-  return r;
-}
-template <int V>
-__device__ __forceinline__ Row<V> row_add(const Row<V> &a, const Row<V> &b) {
-  Row<V> r;
-  if constexpr (V == 1) {
-    r.w = a.w + b.w;
-  } else {
-#pragma unroll
-    for (int i = 0; i < V / 2; ++i)
-      asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.w[i]) : "l"(a.w[i]), "l"(b.w[i]));
-  }
-  return r;
-}
-template <int V>
-__device__ __forceinline__ void row_fma(Row<V> &acc, const Row<V> &a, const Row<V> &b) {
-  if constexpr (V == 1) {
-    acc.w = fmaf(a.w, b.w, acc.w);
-  } else {
-#pragma unroll
-    for (int i = 0; i < V / 2; ++i)
-      asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc.w[i]) : "l"(a.w[i]), "l"(b.w[i]));
-  }
-}
-// A factor row as it is loaded: FP32 columns, or BF16 pairs.
-template <int V, FactorType FT>
-struct RawRow {
-  Row<V> r;
-};
-template <int V>
-struct RawRow<V, FactorType::BF16> {
-  uint32_t w[(V + 1) / 2];
-};
-template <int V, FactorType FT>
-__device__ __forceinline__ Row<V> raw_row(const RawRow<V, FT> &a) {
-  if constexpr (FT == FactorType::F32) {
-    return a.r;
-  } else {
-    // a BF16 value is the upper half of its FP32 value
-    Row<V> r;
-    if constexpr (V == 1) {
-      r.w = __uint_as_float(a.w[0] << 16);
-    } else {
-#pragma unroll
-      for (int i = 0; i < V / 2; ++i)
-        r.w[i] = pack2(__uint_as_float(a.w[i] << 16), __uint_as_float(a.w[i] & 0xFFFF0000u));
-    }
-    return r;
-  }
-}
-// Loaded where on != 0, without a branch; elsewhere the row keeps its value.
-template <int V, FactorType FT>
-__device__ __forceinline__ void ld_row_if(RawRow<V, FT> &a, const char *p, uint32_t on) {
-  if constexpr (FT == FactorType::F32) {
-    if constexpr (V == 1)
-      asm("{\n.reg .pred q;\nsetp.ne.u32 q, %2, 0;\n@q ld.global.nc.f32 %0, [%1];\n}"
-          : "+f"(a.r.w)
-          : "l"(p), "r"(on));
-    else if constexpr (V == 2)
-      asm("{\n.reg .pred q;\nsetp.ne.u32 q, %2, 0;\n@q ld.global.nc.b64 %0, [%1];\n}"
-          : "+l"(a.r.w[0])
-          : "l"(p), "r"(on));
-    else
-      asm("{\n.reg .pred q;\nsetp.ne.u32 q, %3, 0;\n@q ld.global.nc.v2.b64 {%0, %1}, [%2];\n}"
-          : "+l"(a.r.w[0]), "+l"(a.r.w[1])
-          : "l"(p), "r"(on));
-  } else {
-    if constexpr (V == 1)
-      asm("{\n.reg .pred q;\n.reg .b16 h;\nsetp.ne.u32 q, %2, 0;\n@q ld.global.nc.b16 h, [%1];\n"
-          "@q cvt.u32.u16 %0, h;\n}"
-          : "+r"(a.w[0])
-          : "l"(p), "r"(on));
-    else if constexpr (V == 2)
-      asm("{\n.reg .pred q;\nsetp.ne.u32 q, %2, 0;\n@q ld.global.nc.b32 %0, [%1];\n}"
-          : "+r"(a.w[0])
-          : "l"(p), "r"(on));
-    else
-      asm("{\n.reg .pred q;\nsetp.ne.u32 q, %3, 0;\n@q ld.global.nc.v2.b32 {%0, %1}, [%2];\n}"
-          : "+r"(a.w[0]), "+r"(a.w[1])
-          : "l"(p), "r"(on));
-  }
-}
-template <int V, FactorType FT>
-__device__ __forceinline__ void raw_zero(RawRow<V, FT> &a) {
-  if constexpr (FT == FactorType::F32) {
-    a.r = row_zero<V>();
-  } else {
-#pragma unroll
-    for (int i = 0; i < (V + 1) / 2; ++i) a.w[i] = 0u;
-  }
-}
-template <int V, FactorType FT>
-__device__ __forceinline__ void ld_row(RawRow<V, FT> &a, const char *p) {
-  if constexpr (FT == FactorType::F32) {
-    if constexpr (V == 1)
-      asm("ld.global.nc.f32 %0, [%1];" : "=f"(a.r.w) : "l"(p));
-    else if constexpr (V == 2)
-      asm("ld.global.nc.b64 %0, [%1];" : "=l"(a.r.w[0]) : "l"(p));
-    else
-      asm("ld.global.nc.v2.b64 {%0, %1}, [%2];" : "=l"(a.r.w[0]), "=l"(a.r.w[1]) : "l"(p));
-  } else {
-    if constexpr (V == 1)
-      a.w[0] = __ldg(reinterpret_cast<const unsigned short *>(p));
-    else if constexpr (V == 2)
-      asm("ld.global.nc.b32 %0, [%1];" : "=r"(a.w[0]) : "l"(p));
-    else
-      asm("ld.global.nc.v2.b32 {%0, %1}, [%2];" : "=r"(a.w[0]), "=r"(a.w[1]) : "l"(p));
-  }
-}
-template <int V, FactorType FT>
-__device__ __forceinline__ Row<V> ld_row(const char *p) {
-  RawRow<V, FT> a;
-  ld_row<V, FT>(a, p);
-  return raw_row<V, FT>(a);
-}
-__device__ __forceinline__ const char *row_at(const char *base, uint32_t row, uint32_t stride) {
-  return base + (uint64_t)row * stride;
-}
-// The tree's arrays are read once, in order: a miss brings the next units
-// into L2 as well.
-__device__ __forceinline__ uint32_t ld_stream(const uint32_t *p) {
-  uint32_t v;
-  asm("ld.global.nc.L2::256B.b32 %0, [%1];" : "=r"(v) : "l"(p));
-  return v;
-}
-__device__ __forceinline__ float ld_stream(const float *p) {
-  float v;
-  asm("ld.global.nc.L2::256B.f32 %0, [%1];" : "=f"(v) : "l"(p));
-  return v;
-}
-__device__ __forceinline__ uint32_t ld_stream(const uint8_t *p) {
-  uint32_t v;
-  asm("ld.global.nc.L2::256B.u8 %0, [%1];" : "=r"(v) : "l"(p));
-  return v;
-}
-
 // ---------------------------------------------------------------------------
 // Contraction (S > d).
 //
@@ -423,7 +72,7 @@ __device__ __forceinline__ uint32_t ld_stream(const uint8_t *p) {
 // (memo rows, outputs), or multiplied by its own factor row and added to the
 // open node of the level above, in shared memory, and so on up as far as the
 // unit closes. The sums of the nodes that a chunk boundary cuts go to
-// per-chunk head and tail rows (k_chain_groups adds them).
+// per-chunk head and tail rows (sums.cuh adds them).
 //
 // What bounds it: the L1 data pipe and the latency of the gathers behind it,
 // not DRAM. A row of R = 32 columns takes one of its cycles, so a unit takes
@@ -955,59 +604,9 @@ __global__ void k_schedule(WalkArgs a, uint32_t *sched) {
 }
 
 // ---------------------------------------------------------------------------
-// Deterministic accumulation: chain sums of cut nodes, prefix rows, pulls.
+// Cut nodes, prefix rows, pulls.
 // ---------------------------------------------------------------------------
-constexpr uint32_t kChainGroup = 32;  // partials one warp sums per group
 constexpr uint32_t kPullSeg = 256;    // units per pull segment (whole rows) and per piece, at most
-
-struct ChainArgs {
-  const float *span;
-  int span_nlev, ldr, R;
-  int span_lev[kMaxModes];
-  const uint32_t *chains;  // 6 per chain
-  const uint32_t *groups;  // 3 per group
-  uint32_t nchains, ngroups;
-  double *gsum;
-  float *store[kMaxModes];
-  double *out;             // level-0 output rows (output level 0), else nullptr
-  const uint32_t *root_ids;
-};
-
-// Partial k of the chain of a node cut by the boundaries of chunks
-// c_first..c_last: k <= c_last - c_first is the tail of chunk c_first-1+k,
-// the last one the head of chunk c_last (where the node closes).
-__device__ __forceinline__ const float *chain_partial(const ChainArgs &a, int ls, uint32_t c_first,
-                                                      uint32_t c_last, uint32_t k) {
-  const uint32_t ntail = c_last - c_first + 1;
-  const uint32_t c = k < ntail ? c_first - 1 + k : c_last;
-  const int which = k < ntail ? 1 : 0;
-  return a.span + (((size_t)c * a.span_nlev + ls) * 2 + which) * a.ldr;
-}
-
-// One warp per group: its partials summed in chunk order.
-__global__ void k_chain_groups(const __grid_constant__ ChainArgs a) {
-  const uint32_t g = (uint32_t)((blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5);
-  const int lane = threadIdx.x & 31;
-  if (g >= a.ngroups) return;
-  const uint32_t ch = a.groups[3 * (size_t)g], k0 = a.groups[3 * (size_t)g + 1],
-                 cnt = a.groups[3 * (size_t)g + 2];
-  const uint32_t *c = a.chains + 6 * (size_t)ch;
-  const int ls = a.span_lev[c[0]];
-  for (int col = lane; col < a.R; col += 32) {
-    // loads issued eight at a time, added in chunk order
-    double acc = 0.0;
-    uint32_t k = k0;
-    for (; k + 8 <= k0 + cnt; k += 8) {
-      float v[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) v[q] = chain_partial(a, ls, c[2], c[3], k + q)[col];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) acc += (double)v[q];
-    }
-    for (; k < k0 + cnt; ++k) acc += (double)chain_partial(a, ls, c[2], c[3], k)[col];
-    a.gsum[(size_t)g * a.ldr + col] = acc;
-  }
-}
 
 // Sum of n FP64 rows (stride ldr) in index order, column col: loads issued
 // eight at a time.
@@ -1045,36 +644,15 @@ __device__ __forceinline__ void block_ordered_sum(const double *rows, uint64_t n
   __syncthreads();
 }
 
-// A chain's total, stored to the node's memo row and, at level 0 with a
-// root output, to its output row.
-__device__ __forceinline__ void chain_store(const ChainArgs &a, const uint32_t *c, int col, double v) {
-  const int l = (int)c[0];
-  const uint32_t node = c[1];
-  if (a.store[l]) a.store[l][(size_t)node * a.ldr + col] = (float)v;
-  if (l == 0 && a.out) a.out[(size_t)a.root_ids[node] * a.ldr + col] = v;
-}
-
-// Chains of at most kChainShort groups: one warp each, the group sums in
-// order.
-constexpr uint32_t kChainShort = 16;
-__global__ void k_chain_finish(const __grid_constant__ ChainArgs a, const uint32_t *ids, uint32_t n) {
-  const uint32_t i = (uint32_t)((blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5);
-  const int lane = threadIdx.x & 31;
-  if (i >= n) return;
-  const uint32_t *c = a.chains + 6 * (size_t)ids[i];
-  for (int col = lane; col < a.R; col += 32)
-    chain_store(a, c, col, ordered_sum(a.gsum + (size_t)c[4] * a.ldr, c[5], a.ldr, col));
-}
-
-// Longer chains (a skewed root slice cut by thousands of chunks): one block
-// each.
-__global__ void __launch_bounds__(256) k_chain_finish_long(const __grid_constant__ ChainArgs a,
-                                                           const uint32_t *ids) {
-  __shared__ double red[kWarps * 128];
-  __shared__ double tot[128];
-  const uint32_t *c = a.chains + 6 * (size_t)ids[blockIdx.x];
-  block_ordered_sum(a.gsum + (size_t)c[4] * a.ldr, c[5], a.ldr, a.R, red, tot);
-  for (int col = threadIdx.x; col < a.R; col += blockDim.x) chain_store(a, c, col, tot[col]);
+// The nodes that chunk boundaries cut: cut[k * nchunks + c] = 1 + the node of
+// the k-th spanned level that began before chunk c, else 0.
+__global__ void k_cut_nodes(WalkArgs a, uint32_t *cut) {
+  const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= a.nchunks) return;
+  const uint32_t *sc = a.sched + (size_t)c * (a.S + 1);
+  for (int l = 0; l < a.S; ++l)
+    if (a.span_lev[l] >= 0)
+      cut[(size_t)a.span_lev[l] * a.nchunks + c] = (sc[a.S] >> l) & 1u ? sc[l] + 1u : 0u;
 }
 
 // parent[c] = p for the children c of every node p (fptr of the parent level).
@@ -1472,7 +1050,7 @@ void to_device(DevBuf<T> &dst, const std::vector<T> &h, cudaStream_t s) {
   ADATM_CUDA(cudaStreamSynchronize(s));
 }
 
-// Slots and chains of a contraction: the levels whose cut nodes are summed
+// Span slots and chains of a contraction: the levels whose cut nodes are summed
 // over chunks (stored levels, and level 0 when it is the output), and for
 // each node a chunk boundary cuts, the run of chunks it spans. Contractions
 // below the root also store their level-d sums for the pull or the scatter.
@@ -1503,52 +1081,16 @@ void prepare_spans(TreeWalk &w, cudaStream_t s) {
   for (int l = 0; l < kMaxModes; ++l) w.span_lev[l] = -1;
   for (int l = 0; l < S; ++l)
     if (w.store[l] != nullptr || (l == 0 && d == 0)) w.span_lev[l] = w.span_nlev++;
-  w.nchains = w.ngroups = 0;
   if (w.nchunks == 0 || w.span_nlev == 0) return;
   w.span.alloc((size_t)w.nchunks * w.span_nlev * 2 * w.ldr);
-  const std::vector<uint32_t> sc = to_host(w.sched.get(), (size_t)w.nchunks * (S + 1), s);
-  std::vector<uint32_t> chains, groups;
-  const size_t st = (size_t)S + 1;
-  for (int l = 0; l < S; ++l) {
-    if (w.span_lev[l] < 0) continue;
-    uint32_t ch = 1;
-    while (ch < w.nchunks) {
-      if (!((sc[ch * st + S] >> l) & 1u)) {
-        ++ch;
-        continue;
-      }
-      const uint32_t node = sc[ch * st + l];
-      uint32_t last = ch;
-      while (last + 1 < w.nchunks && ((sc[(last + 1) * st + S] >> l) & 1u) &&
-             sc[(last + 1) * st + l] == node)
-        ++last;
-      const uint32_t npart = (last - ch + 1) + 1;
-      const uint32_t id = (uint32_t)(chains.size() / 6);
-      const uint32_t g0 = (uint32_t)(groups.size() / 3);
-      const uint32_t ng = (npart + kChainGroup - 1) / kChainGroup;
-      for (uint32_t k0 = 0; k0 < npart; k0 += kChainGroup) {
-        groups.push_back(id);
-        groups.push_back(k0);
-        groups.push_back(std::min(kChainGroup, npart - k0));
-      }
-      const uint32_t row[6] = {(uint32_t)l, node, ch, last, g0, ng};
-      chains.insert(chains.end(), row, row + 6);
-      ch = last + 1;
-    }
-  }
-  w.nchains = (uint32_t)(chains.size() / 6);
-  w.ngroups = (uint32_t)(groups.size() / 3);
-  // short chains first (a warp each), then long ones (a block each)
-  std::vector<uint32_t> ids;
-  for (uint32_t i = 0; i < w.nchains; ++i)
-    if (chains[6 * (size_t)i + 5] <= kChainShort) ids.push_back(i);
-  w.nshort = (uint32_t)ids.size();
-  for (uint32_t i = 0; i < w.nchains; ++i)
-    if (chains[6 * (size_t)i + 5] > kChainShort) ids.push_back(i);
-  to_device(w.chain_ids, ids, s);
-  to_device(w.chains, chains, s);
-  to_device(w.groups, groups, s);
-  w.gsum.alloc((size_t)std::max<uint32_t>(w.ngroups, 1) * w.ldr);
+  ADATM_CUDA(cudaMemsetAsync(w.span.get(), 0, w.span.bytes(), s));  // padding columns stay zero
+  DevBuf<uint32_t> cut((size_t)w.span_nlev * w.nchunks);
+  k_cut_nodes<<<(w.nchunks + 255) / 256, 256, 0, s>>>(make_args(w, nullptr, nullptr), cut.get());
+  ADATM_LAUNCH();
+  int level_of[kMaxModes];
+  for (int l = 0; l < S; ++l)
+    if (w.span_lev[l] >= 0) level_of[w.span_lev[l]] = l;
+  span_prepare(w.sums, cut.get(), w.span_nlev, level_of, w.nchunks, w.ldr, s);
 }
 
 // The pull of level d = w.out: units (level-d nodes) in a stable order by
@@ -1691,35 +1233,12 @@ void launch_pull(const TreeWalk &w, const LevelFactors &f, FactorType ft, const 
   }
 }
 
-void launch_chains(const TreeWalk &w, double *out, cudaStream_t s) {
-  if (w.nchains == 0) return;
-  ChainArgs a;
-  a.span = w.span.get();
-  a.span_nlev = w.span_nlev;
-  a.ldr = w.ldr;
-  a.R = w.R;
-  for (int l = 0; l < kMaxModes; ++l) {
-    a.span_lev[l] = w.span_lev[l];
-    a.store[l] = w.store[l];
-  }
-  a.chains = w.chains.get();
-  a.groups = w.groups.get();
-  a.nchains = w.nchains;
-  a.ngroups = w.ngroups;
-  a.gsum = w.gsum.get();
-  a.out = w.out == 0 ? out : nullptr;
-  a.root_ids = w.csf->fids[0].get();
-  k_chain_groups<<<(unsigned)(((uint64_t)w.ngroups * 32 + 255) / 256), 256, 0, s>>>(a);
-  ADATM_LAUNCH();
-  if (w.nshort) {
-    k_chain_finish<<<(unsigned)(((uint64_t)w.nshort * 32 + 255) / 256), 256, 0, s>>>(
-        a, w.chain_ids.get(), w.nshort);
-    ADATM_LAUNCH();
-  }
-  if (w.nchains > w.nshort) {
-    k_chain_finish_long<<<w.nchains - w.nshort, 256, 0, s>>>(a, w.chain_ids.get() + w.nshort);
-    ADATM_LAUNCH();
-  }
+void launch_sums(const TreeWalk &w, double *out, cudaStream_t s) {
+  SpanTarget t;
+  for (int l = 0; l < kMaxModes; ++l) t.store[l] = w.store[l];
+  t.out = w.out == 0 ? out : nullptr;
+  t.out_ids = w.csf->fids[0].get();
+  span_launch<float>(w.sums, w.span.get(), w.span_nlev, w.R, w.ldr, t, s);
 }
 
 }  // namespace
@@ -1820,7 +1339,7 @@ void walk_launch(const TreeWalk &w, const LevelFactors &f, FactorType ft, double
       if (leaf) launch_contract<FactorType::BF16, true>(wk, w.fold, a, w.resident, s);
       else launch_contract<FactorType::BF16, false>(wk, w.fold, a, w.resident, s);
     }
-    launch_chains(w, out, s);
+    launch_sums(w, out, s);
     if (w.scatter) walk_launch(*w.scatter, f, ft, out, s);
     else if (w.out > 0) launch_pull(w, f, ft, w.level_rows.get(), out, s);
   } else {
@@ -1841,7 +1360,7 @@ int walk_kernels(const TreeWalk &w) {
   int k = 0;
   if (w.src > w.out) {
     k += 1;                                            // the contraction
-    if (w.nchains) k += 1 + (w.nshort ? 1 : 0) + (w.nchains > w.nshort ? 1 : 0);  // chain sums
+    k += span_kernels(w.sums);                         // the cut nodes' sums
   }
   if (w.deterministic && w.nsegs) k += w.out + 1 + (w.nlong ? 1 : 0);  // prefix levels, pull, pieces
   if (!w.deterministic && w.src == w.out) k += 1;      // the scatter

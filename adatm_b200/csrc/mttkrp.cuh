@@ -25,6 +25,7 @@
 #include <memory>
 
 #include "csf_build.cuh"
+#include "sums.cuh"
 
 namespace adatm {
 
@@ -63,9 +64,8 @@ struct TreeWalk {
   DevBuf<uint32_t> hot_rows;
   // Nodes that chunk boundaries cut (contractions, every mode): their
   // partial sums go to per-chunk rows (span) and are summed per node in
-  // chunk order and in FP64 (chains, in groups of kChainGroup partials), so
-  // a node spanning thousands of chunks (a skewed root slice) takes no long
-  // chain of FP32 atomics. Deterministic accumulation additionally pulls
+  // chunk order and in FP64 (sums), so a node spanning thousands of chunks (a
+  // skewed root slice) takes no long chain of FP32 atomics. Deterministic accumulation additionally pulls
   // scatters, and the output of contractions below the root, per output row
   // in the order of a stable sort by output row (segments of whole rows, long
   // rows split into pieces summed in order): no float atomics anywhere, so
@@ -74,13 +74,7 @@ struct TreeWalk {
   int span_nlev = 0;
   int span_lev[kMaxModes] = {-1, -1, -1, -1, -1, -1, -1, -1};
   DevBuf<float> span;                // nchunks x span_nlev x 2 x ldr
-  DevBuf<uint32_t> chains;           // per chain: level, node, first boundary chunk, last chunk,
-                                     // first group, groups
-  DevBuf<uint32_t> groups;           // per group: chain, first partial, partials
-  DevBuf<double> gsum;               // per group: its sum (ldr)
-  uint32_t nchains = 0, ngroups = 0;
-  DevBuf<uint32_t> chain_ids;        // chains of few groups first (nshort), then long ones
-  uint32_t nshort = 0;
+  SpanSums sums;
   DevBuf<float> level_rows;          // contraction below the root: level-d node sums
   std::unique_ptr<TreeWalk> scatter; // and, with atomics, their scatter into the output rows
   // pull scatter of level `out` (deterministic scatters and contractions below the root)
