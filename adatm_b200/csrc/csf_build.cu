@@ -16,6 +16,7 @@
 //     node opening at n (or n itself for l = N-2).
 // No kernel waits on another block; every phase is a separate launch.
 #include <cmath>
+#include <utility>
 #include <vector>
 
 #include "csf_build.cuh"
@@ -268,18 +269,14 @@ struct SortBufs {
   uint32_t *order = nullptr;
 };
 
-// Sort keys (packed from `coo` under `spec`) stably; result in b.keys/b.order.
+// Sort the keys of n units (levels idx packed under `spec`) stably; result in
+// b.keys/b.order.
 template <int W>
-void sort_keys(const DevCoo &coo, const uint64_t *perm, const KeySpec &spec, SortBufs<W> &b,
-               cudaStream_t s) {
-  const uint64_t n = coo.nnz;
+void sort_keys(const IdxPtrs &ip, uint64_t n, const KeySpec &spec, SortBufs<W> &b, cudaStream_t s) {
   b.k0.alloc(n);
   b.k1.alloc(n);
   b.o0.alloc(n);
   b.o1.alloc(n);
-  IdxPtrs ip;
-  for (int l = 0; l < kMaxModes; ++l) ip.p[l] = nullptr;
-  for (int l = 0; l < coo.nmodes; ++l) ip.p[l] = coo.idx[perm[l]].get();
   const unsigned blocks = (unsigned)((n + 255) / 256);
   k_pack<W><<<blocks, 256, 0, s>>>(ip, spec, n, b.k0.get(), b.o0.get());
   ADATM_LAUNCH();
@@ -304,6 +301,19 @@ void sort_keys(const DevCoo &coo, const uint64_t *perm, const KeySpec &spec, Sor
   }
   b.keys = kin;
   b.order = oin;
+}
+
+template <int W>
+void sort_keys(const DevCoo &coo, const uint64_t *perm, const KeySpec &spec, SortBufs<W> &b,
+               cudaStream_t s) {
+  IdxPtrs ip = {};
+  for (int l = 0; l < coo.nmodes; ++l) ip.p[l] = coo.idx[perm[l]].get();
+  sort_keys<W>(ip, coo.nnz, spec, b, s);
+}
+
+__global__ void k_narrow_keys(const Key<1> *keys, uint64_t n, uint32_t *out) {
+  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) out[i] = (uint32_t)keys[i].w[0];
 }
 
 // ---------------------------------------------------------------------------
@@ -846,6 +856,22 @@ void csf_count(const DevCoo &coo, const uint64_t *perm, uint64_t *nfibs, cudaStr
     case 2: count_w<2>(coo, perm, spec, nfibs, s); break;
     default: count_w<3>(coo, perm, spec, nfibs, s); break;
   }
+}
+
+void sort_by_row(const uint32_t *row, uint64_t n, uint64_t nrows, DevBuf<uint32_t> &perm,
+                 DevBuf<uint32_t> &sorted, cudaStream_t s) {
+  if (n == 0) return;
+  const uint64_t dims[1] = {nrows}, order[1] = {0};
+  const KeySpec spec = make_key_spec(1, dims, order);
+  IdxPtrs ip = {};
+  ip.p[0] = row;
+  SortBufs<1> b;
+  sort_keys<1>(ip, n, spec, b, s);
+  sorted.alloc(n);
+  k_narrow_keys<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(b.keys, n, sorted.get());
+  ADATM_LAUNCH();
+  ADATM_CUDA(cudaStreamSynchronize(s));
+  perm = std::move(b.order == b.o0.get() ? b.o0 : b.o1);
 }
 
 void csf_download(const DevCsf &c, HostCsfArrays &h, cudaStream_t s) {

@@ -74,6 +74,11 @@ void csf_build(const DevCoo &coo, const uint64_t *perm, DevCsf &out, cudaStream_
 // building the arrays. nfibs[N-1] = nnz.
 void csf_count(const DevCoo &coo, const uint64_t *perm, uint64_t *nfibs, cudaStream_t s);
 
+// Stable sort of units 0 .. n-1 by row[unit] (rows below nrows): perm[j] is the
+// j-th unit, sorted[j] its row.
+void sort_by_row(const uint32_t *row, uint64_t n, uint64_t nrows, DevBuf<uint32_t> &perm,
+                 DevBuf<uint32_t> &sorted, cudaStream_t s);
+
 // Copy a device CSF into host arrays in the reference layout (64-bit).
 struct HostCsfArrays {
   std::vector<std::vector<uint64_t>> fptr, fids;

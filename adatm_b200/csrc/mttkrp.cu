@@ -3,6 +3,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "mttkrp.cuh"
 #include "rows.cuh"
 
 namespace adatm {
@@ -604,46 +605,8 @@ __global__ void k_schedule(WalkArgs a, uint32_t *sched) {
 }
 
 // ---------------------------------------------------------------------------
-// Cut nodes, prefix rows, pulls.
+// Cut nodes.
 // ---------------------------------------------------------------------------
-constexpr uint32_t kPullSeg = 256;    // units per pull segment (whole rows) and per piece, at most
-
-// Sum of n FP64 rows (stride ldr) in index order, column col: loads issued
-// eight at a time.
-__device__ __forceinline__ double ordered_sum(const double *rows, uint64_t n, int ldr, int col) {
-  double acc = 0.0;
-  uint64_t k = 0;
-  for (; k + 8 <= n; k += 8) {
-    double v[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) v[q] = rows[(k + q) * ldr + col];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) acc += v[q];
-  }
-  for (; k < n; ++k) acc += rows[k * ldr + col];
-  return acc;
-}
-
-// Sum of n FP64 rows in index order by a whole block: warp w sums the w-th
-// of 8 contiguous ranges, then the 8 range sums are added in order. The
-// split depends only on n, so the result does not depend on scheduling.
-__device__ __forceinline__ void block_ordered_sum(const double *rows, uint64_t n, int ldr, int R,
-                                                  double *red /* kWarps x R */, double *out_col) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint64_t per = (n + kWarps - 1) / kWarps;
-  const uint64_t b = min(n, (uint64_t)warp * per), e = min(n, b + per);
-  for (int col = lane; col < R; col += 32)
-    red[warp * R + col] = ordered_sum(rows + b * ldr, e - b, ldr, col);
-  __syncthreads();
-  if (warp == 0)
-    for (int col = lane; col < R; col += 32) {
-      double acc = 0.0;
-      for (int w = 0; w < kWarps; ++w) acc += red[w * R + col];
-      out_col[col] = acc;
-    }
-  __syncthreads();
-}
-
 // The nodes that chunk boundaries cut: cut[k * nchunks + c] = 1 + the node of
 // the k-th spanned level that began before chunk c, else 0.
 __global__ void k_cut_nodes(WalkArgs a, uint32_t *cut) {
@@ -653,123 +616,6 @@ __global__ void k_cut_nodes(WalkArgs a, uint32_t *cut) {
   for (int l = 0; l < a.S; ++l)
     if (a.span_lev[l] >= 0)
       cut[(size_t)a.span_lev[l] * a.nchunks + c] = (sc[a.S] >> l) & 1u ? sc[l] + 1u : 0u;
-}
-
-// parent[c] = p for the children c of every node p (fptr of the parent level).
-__global__ void k_fill_parent(const uint32_t *fptr, uint64_t nparent, uint32_t *parent) {
-  for (uint64_t p = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; p < nparent;
-       p += (uint64_t)gridDim.x * blockDim.x)
-    for (uint32_t c = fptr[p]; c < fptr[p + 1]; ++c) parent[c] = (uint32_t)p;
-}
-
-// Prefix rows of one level: P_l[n] = P_{l-1}[parent(n)] * U_l[fids_l[n]]
-// (P_0[n] = U_0[fids_0[n]]); padding columns are zero.
-template <FactorType FT>
-__global__ void k_prefix_level(const void *U, const uint32_t *fids, const uint32_t *parent,
-                               const float *prev, uint64_t n, int R, int ldr, float *out) {
-  const int q = ldr / 4;
-  const uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (e >= n * (uint64_t)q) return;
-  const uint64_t node = e / q;
-  const int col = 4 * (int)(e % q);
-  const fv<4> u = ld_factor<4, FT>(U, fids[node], ldr, col, col < R);
-  float4 r = make_float4(u.x[0], u.x[1], u.x[2], u.x[3]);
-  if (prev) {
-    const float4 p = *reinterpret_cast<const float4 *>(prev + (size_t)parent[node] * ldr + col);
-    r = make_float4(r.x * p.x, r.y * p.y, r.z * p.z, r.w * p.w);
-  }
-  *reinterpret_cast<float4 *>(out + node * ldr + col) = r;
-}
-
-struct PullArgs {
-  int d, R, ldr;
-  const uint32_t *perm, *prow, *pparent, *segs;
-  uint32_t nsegs;
-  const float *vals;      // leaf values (leaf source)
-  const float *src_rows;  // node rows of level d (row source)
-  const float *prefix;    // P_{d-1} rows (d >= 1)
-  double *out;
-  double *piece_sum;
-};
-
-// Pull scatter: one warp per segment of units sorted by output row; each
-// unit's contribution src(u) * P_{d-1}[parent(u)] is added in that order and
-// a row is stored once, when its last unit is done (whole rows), or into its
-// piece's slot (long rows, summed in order by k_piece_sum).
-template <int V, bool LEAF>
-__global__ void __launch_bounds__(256) k_pull(const __grid_constant__ PullArgs a) {
-  __shared__ uint4 stage[kWarps][kBatch];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int col = lane * V;
-  const bool act = col < a.R;
-  constexpr int SB = 8;
-  for (uint32_t sg = blockIdx.x * kWarps + warp; sg < a.nsegs; sg += gridDim.x * kWarps) {
-    const uint32_t jb = a.segs[3 * (size_t)sg], je = a.segs[3 * (size_t)sg + 1],
-                   slot = a.segs[3 * (size_t)sg + 2];
-    double acc[V];
-#pragma unroll
-    for (int i = 0; i < V; ++i) acc[i] = 0.0;
-    uint32_t cur = a.prow[jb];
-    auto flush = [&](uint32_t row) {
-      if (!act) return;
-      double *p = (slot == 0xFFFFFFFFu ? a.out + (size_t)row * a.ldr : a.piece_sum + (size_t)slot * a.ldr) + col;
-#pragma unroll
-      for (int i = 0; i < V; ++i) p[i] = acc[i];
-    };
-    for (uint32_t j0 = jb; j0 < je; j0 += kBatch) {
-      const int cnt = (int)min((uint32_t)kBatch, je - j0);
-      if (lane < cnt) {
-        const uint32_t u = a.perm[j0 + lane];
-        const float v = LEAF ? a.vals[u] : 0.f;
-        stage[warp][lane] = make_uint4(u, a.prow[j0 + lane], a.d >= 1 ? a.pparent[j0 + lane] : 0u,
-                                       __float_as_uint(v));
-      }
-      __syncwarp();
-      for (int k0 = 0; k0 < cnt; k0 += SB) {
-        fv<V> x[SB];
-#pragma unroll
-        for (int q = 0; q < SB; ++q) {
-          const int k = k0 + q;
-          const bool ok = k < cnt;
-          const uint4 e = stage[warp][ok ? k : 0];
-          fv<V> t;
-          if constexpr (LEAF) t = fv_fill<V>(__uint_as_float(e.w));
-          else t = ld_rows<V>(a.src_rows, e.x, a.ldr, col, ok && act);
-          if (a.d >= 1) t = fv_mul(t, ld_rows<V>(a.prefix, e.z, a.ldr, col, ok && act));
-          x[q] = t;
-        }
-#pragma unroll
-        for (int q = 0; q < SB; ++q) {
-          const int k = k0 + q;
-          if (k < cnt) {
-            const uint32_t row = stage[warp][k].y;
-            if (row != cur) {
-              flush(cur);
-#pragma unroll
-              for (int i = 0; i < V; ++i) acc[i] = 0.0;
-              cur = row;
-            }
-#pragma unroll
-            for (int i = 0; i < V; ++i) acc[i] += (double)x[q].x[i];
-          }
-        }
-      }
-      __syncwarp();
-    }
-    flush(cur);
-  }
-}
-
-// One block per long row: its pieces summed in order.
-__global__ void __launch_bounds__(256) k_piece_sum(const uint32_t *pieces, const double *piece_sum,
-                                                   int R, int ldr, double *out) {
-  __shared__ double red[kWarps * 128];
-  __shared__ double tot[128];
-  const uint32_t i = blockIdx.x;
-  const uint32_t row = pieces[3 * (size_t)i], p0 = pieces[3 * (size_t)i + 1],
-                 np = pieces[3 * (size_t)i + 2];
-  block_ordered_sum(piece_sum + (size_t)p0 * ldr, np, ldr, R, red, tot);
-  for (int col = threadIdx.x; col < R; col += blockDim.x) out[(size_t)row * ldr + col] = tot[col];
 }
 
 WalkArgs make_args(const TreeWalk &w, const LevelFactors *f, double *out) {
@@ -952,14 +798,6 @@ void launch_scatter(int w, const WalkArgs &a, unsigned blocks, cudaStream_t s) {
   ADATM_LAUNCH();
 }
 
-// Contraction: columns per lane (32 lanes cover R).
-int vec_for_rank(int R) {
-  if (R <= 32) return 1;
-  if (R <= 64) return 2;
-  if (R <= 128) return 4;
-  throw BadInput("rank above 128 is not supported by the GPU kernels");
-}
-
 }  // namespace
 
 // As many walkers as cover the rank at four columns (one 16-byte load) per lane.
@@ -1030,25 +868,9 @@ void set_walk_attributes() {
 }
 
 // ---------------------------------------------------------------------------
-// Deterministic walks: preparation and launch.
+// Preparation and launch.
 // ---------------------------------------------------------------------------
 namespace {
-
-template <typename T>
-std::vector<T> to_host(const T *dev, size_t n, cudaStream_t s) {
-  std::vector<T> h(n);
-  if (n) ADATM_CUDA(cudaMemcpyAsync(h.data(), dev, n * sizeof(T), cudaMemcpyDeviceToHost, s));
-  ADATM_CUDA(cudaStreamSynchronize(s));
-  return h;
-}
-
-template <typename T>
-void to_device(DevBuf<T> &dst, const std::vector<T> &h, cudaStream_t s) {
-  dst.alloc(std::max<size_t>(h.size(), 1));
-  if (!h.empty())
-    ADATM_CUDA(cudaMemcpyAsync(dst.get(), h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, s));
-  ADATM_CUDA(cudaStreamSynchronize(s));
-}
 
 // Span slots and chains of a contraction: the levels whose cut nodes are summed
 // over chunks (stored levels, and level 0 when it is the output), and for
@@ -1063,9 +885,7 @@ void prepare_spans(TreeWalk &w, cudaStream_t s) {
     w.level_rows.alloc((size_t)std::max<uint64_t>(c.nfibs[d], 1) * w.ldr);
     ADATM_CUDA(cudaMemsetAsync(w.level_rows.get(), 0, w.level_rows.bytes(), s));
     w.store[d] = w.level_rows.get();
-    if (w.deterministic) {
-      w.pull = true;
-    } else {
+    if (!w.deterministic) {
       w.scatter = std::make_unique<TreeWalk>();
       TreeWalk &t = *w.scatter;
       t.csf = w.csf;
@@ -1091,146 +911,6 @@ void prepare_spans(TreeWalk &w, cudaStream_t s) {
   for (int l = 0; l < S; ++l)
     if (w.span_lev[l] >= 0) level_of[w.span_lev[l]] = l;
   span_prepare(w.sums, cut.get(), w.span_nlev, level_of, w.nchunks, w.ldr, s);
-}
-
-// The pull of level d = w.out: units (level-d nodes) in a stable order by
-// output row, their parents, segments of whole rows and pieces of long rows,
-// the parent arrays and prefix buffers of the levels above.
-void det_prepare_pull(TreeWalk &w, cudaStream_t s) {
-  const DevCsf &c = *w.csf;
-  const int d = w.out;
-  const uint64_t n = c.nfibs[d];
-  const uint64_t rows = c.dims[c.dim_perm[d]];
-  const std::vector<uint32_t> fid = to_host(c.fids[d].get(), n, s);
-  std::vector<uint32_t> par;
-  if (d >= 1) {
-    const std::vector<uint32_t> fp = to_host(c.fptr[d - 1].get(), c.nfibs[d - 1] + 1, s);
-    par.assign(n, 0);
-    for (uint64_t p = 0; p < c.nfibs[d - 1]; ++p)
-      for (uint32_t u = fp[p]; u < fp[p + 1] && u < n; ++u) par[u] = (uint32_t)p;
-  }
-  // stable counting sort by output row
-  std::vector<uint64_t> start(rows + 1, 0);
-  for (uint64_t u = 0; u < n; ++u) ++start[fid[u] + 1];
-  for (uint64_t r = 0; r < rows; ++r) start[r + 1] += start[r];
-  std::vector<uint32_t> perm(n), prow(n), pparent(d >= 1 ? n : 0);
-  {
-    std::vector<uint64_t> pos(start.begin(), start.end() - 1);
-    for (uint64_t u = 0; u < n; ++u) {
-      const uint64_t j = pos[fid[u]]++;
-      perm[j] = (uint32_t)u;
-      prow[j] = fid[u];
-      if (d >= 1) pparent[j] = par[u];
-    }
-  }
-  // segments: whole rows packed up to `seg` units (kPullSeg, shorter for
-  // small levels so the segments still fill the device); longer rows in pieces
-  uint64_t seg = kPullSeg;
-  while (seg > 32 && n / seg < 148ull * 32) seg /= 2;
-  std::vector<uint32_t> segs, pieces;
-  uint32_t npieces = 0;
-  uint64_t seg_start = 0, seg_len = 0;
-  auto close_seg = [&](uint64_t end) {
-    if (seg_len > 0) {
-      segs.push_back((uint32_t)seg_start);
-      segs.push_back((uint32_t)end);
-      segs.push_back(0xFFFFFFFFu);
-    }
-    seg_start = end;
-    seg_len = 0;
-  };
-  for (uint64_t r = 0; r < rows; ++r) {
-    const uint64_t b = start[r], cnt = start[r + 1] - b;
-    if (cnt == 0) continue;
-    if (cnt > seg) {
-      close_seg(b);
-      const uint32_t np = (uint32_t)((cnt + seg - 1) / seg);
-      pieces.push_back((uint32_t)r);
-      pieces.push_back(npieces);
-      pieces.push_back(np);
-      for (uint32_t q = 0; q < np; ++q) {
-        segs.push_back((uint32_t)(b + (uint64_t)q * seg));
-        segs.push_back((uint32_t)std::min<uint64_t>(b + (uint64_t)(q + 1) * seg, b + cnt));
-        segs.push_back(npieces + q);
-      }
-      npieces += np;
-      seg_start = b + cnt;
-      continue;
-    }
-    if (seg_len + cnt > seg) close_seg(b);
-    seg_len += cnt;
-  }
-  close_seg(n);
-  w.nsegs = (uint32_t)(segs.size() / 3);
-  w.nlong = (uint32_t)(pieces.size() / 3);
-  w.npieces = npieces;
-  to_device(w.perm, perm, s);
-  to_device(w.prow, prow, s);
-  to_device(w.pparent, pparent, s);
-  to_device(w.segs, segs, s);
-  to_device(w.pieces, pieces, s);
-  w.piece_sum.alloc((size_t)std::max<uint32_t>(npieces, 1) * w.ldr);
-  // parents and prefix rows of levels 1..d-1
-  uint64_t maxf = 1;
-  for (int l = 0; l < d; ++l) maxf = std::max<uint64_t>(maxf, c.nfibs[l]);
-  for (int l = 1; l < d; ++l) {
-    w.parent[l].alloc(std::max<uint64_t>(c.nfibs[l], 1));
-    const uint64_t np = c.nfibs[l - 1];
-    if (np == 0) continue;
-    k_fill_parent<<<(unsigned)std::min<uint64_t>((np + 255) / 256, 65535), 256, 0, s>>>(
-        c.fptr[l - 1].get(), np, w.parent[l].get());
-    ADATM_LAUNCH();
-  }
-  if (d >= 1) w.prefix[0].alloc(maxf * w.ldr);
-  if (d >= 2) w.prefix[1].alloc(maxf * w.ldr);
-  ADATM_CUDA(cudaStreamSynchronize(s));
-}
-
-template <FactorType FT>
-void launch_prefix(const TreeWalk &w, const LevelFactors &f, cudaStream_t s) {
-  const DevCsf &c = *w.csf;
-  for (int l = 0; l < w.out; ++l) {
-    const uint64_t n = c.nfibs[l];
-    if (n == 0) continue;
-    const uint64_t thr = n * (uint64_t)(w.ldr / 4);
-    k_prefix_level<FT><<<(unsigned)((thr + 255) / 256), 256, 0, s>>>(
-        f.U[l], c.fids[l].get(), l ? w.parent[l].get() : nullptr,
-        l ? w.prefix[(l - 1) & 1].get() : nullptr, n, w.R, w.ldr, w.prefix[l & 1].get());
-    ADATM_LAUNCH();
-  }
-}
-
-void launch_pull(const TreeWalk &w, const LevelFactors &f, FactorType ft, const float *rows,
-                 double *out, cudaStream_t s) {
-  if (w.nsegs == 0) return;
-  if (ft == FactorType::F32) launch_prefix<FactorType::F32>(w, f, s);
-  else launch_prefix<FactorType::BF16>(w, f, s);
-  PullArgs a;
-  a.d = w.out;
-  a.R = w.R;
-  a.ldr = w.ldr;
-  a.perm = w.perm.get();
-  a.prow = w.prow.get();
-  a.pparent = w.pparent.get();
-  a.segs = w.segs.get();
-  a.nsegs = w.nsegs;
-  a.vals = w.csf->vals32.get();
-  a.src_rows = rows;
-  a.prefix = w.out >= 1 ? w.prefix[(w.out - 1) & 1].get() : nullptr;
-  a.out = out;
-  a.piece_sum = w.piece_sum.get();
-  const bool leaf = rows == nullptr;
-  const unsigned blocks = (w.nsegs + kWarps - 1) / kWarps;
-  switch (vec_for_rank(w.R)) {
-    case 1: leaf ? k_pull<1, true><<<blocks, 256, 0, s>>>(a) : k_pull<1, false><<<blocks, 256, 0, s>>>(a); break;
-    case 2: leaf ? k_pull<2, true><<<blocks, 256, 0, s>>>(a) : k_pull<2, false><<<blocks, 256, 0, s>>>(a); break;
-    default: leaf ? k_pull<4, true><<<blocks, 256, 0, s>>>(a) : k_pull<4, false><<<blocks, 256, 0, s>>>(a); break;
-  }
-  ADATM_LAUNCH();
-  if (w.nlong) {
-    k_piece_sum<<<w.nlong, 256, 0, s>>>(w.pieces.get(), w.piece_sum.get(), w.R, w.ldr, out);
-    ADATM_LAUNCH();
-  }
 }
 
 void launch_sums(const TreeWalk &w, double *out, cudaStream_t s) {
@@ -1315,9 +995,11 @@ void walk_prepare(TreeWalk &w, cudaStream_t s) {
   WalkArgs a = make_args(w, nullptr, nullptr);
   k_schedule<<<(w.nchunks + 255) / 256, 256, 0, s>>>(a, w.sched.get());
   ADATM_LAUNCH();
-  w.pull = w.deterministic && w.src == w.out;
   if (w.src > w.out) prepare_spans(w, s);
-  if (w.pull) det_prepare_pull(w, s);
+  if (w.deterministic && (w.src == w.out || w.out > 0)) {
+    w.pull = std::make_unique<PullWalk>();
+    pull_prepare(*w.pull, c, w.out, w.src == w.out && w.src == w.nmodes - 1, w.R, w.ldr, s);
+  }
   if (!w.deterministic && w.src == w.out && w.nunits >= kHotMin) find_hot_rows(w, s);
 }
 
@@ -1325,7 +1007,7 @@ void walk_launch(const TreeWalk &w, const LevelFactors &f, FactorType ft, double
                  cudaStream_t s) {
   if (w.nchunks == 0) return;
   if (w.deterministic && w.src == w.out) {
-    launch_pull(w, f, ft, w.src == w.nmodes - 1 ? nullptr : w.src_rows, out, s);
+    pull_launch(*w.pull, f.U, ft, w.src_rows, out, s);
     return;
   }
   const WalkArgs a = make_args(w, &f, w.src > w.out && w.out > 0 ? nullptr : out);
@@ -1341,7 +1023,7 @@ void walk_launch(const TreeWalk &w, const LevelFactors &f, FactorType ft, double
     }
     launch_sums(w, out, s);
     if (w.scatter) walk_launch(*w.scatter, f, ft, out, s);
-    else if (w.out > 0) launch_pull(w, f, ft, w.level_rows.get(), out, s);
+    else if (w.pull) pull_launch(*w.pull, f.U, ft, w.level_rows.get(), out, s);
   } else {
     const unsigned blocks = (unsigned)((w.nchunks + kWarps - 1) / kWarps);
     const int lanes = lanes_for_rank(w.R);
@@ -1362,7 +1044,7 @@ int walk_kernels(const TreeWalk &w) {
     k += 1;                                            // the contraction
     k += span_kernels(w.sums);                         // the cut nodes' sums
   }
-  if (w.deterministic && w.nsegs) k += w.out + 1 + (w.nlong ? 1 : 0);  // prefix levels, pull, pieces
+  if (w.pull) k += pull_kernels(*w.pull);
   if (!w.deterministic && w.src == w.out) k += 1;      // the scatter
   if (w.scatter) k += walk_kernels(*w.scatter);
   return k;

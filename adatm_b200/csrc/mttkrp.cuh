@@ -25,11 +25,10 @@
 #include <memory>
 
 #include "csf_build.cuh"
+#include "pull.cuh"
 #include "sums.cuh"
 
 namespace adatm {
-
-enum class FactorType : int { F32 = 0, BF16 = 1 };
 
 // Factor row matrices of one tree, in level order (U[l] belongs to mode
 // dim_perm[l]); fp32 or bf16 with leading dimension ldr.
@@ -65,11 +64,10 @@ struct TreeWalk {
   // Nodes that chunk boundaries cut (contractions, every mode): their
   // partial sums go to per-chunk rows (span) and are summed per node in
   // chunk order and in FP64 (sums), so a node spanning thousands of chunks (a
-  // skewed root slice) takes no long chain of FP32 atomics. Deterministic accumulation additionally pulls
-  // scatters, and the output of contractions below the root, per output row
-  // in the order of a stable sort by output row (segments of whole rows, long
-  // rows split into pieces summed in order): no float atomics anywhere, so
-  // repeated runs agree bit for bit.
+  // skewed root slice) takes no long chain of FP32 atomics. Deterministic accumulation
+  // pulls scatters, and the output of contractions below the root, per output
+  // row in the order of a stable sort by output row: no float atomics
+  // anywhere, so repeated runs agree bit for bit.
   bool deterministic = false;
   int span_nlev = 0;
   int span_lev[kMaxModes] = {-1, -1, -1, -1, -1, -1, -1, -1};
@@ -77,15 +75,7 @@ struct TreeWalk {
   SpanSums sums;
   DevBuf<float> level_rows;          // contraction below the root: level-d node sums
   std::unique_ptr<TreeWalk> scatter; // and, with atomics, their scatter into the output rows
-  // pull scatter of level `out` (deterministic scatters and contractions below the root)
-  bool pull = false;
-  DevBuf<uint32_t> parent[kMaxModes];  // parent node of every node of levels 1..out
-  DevBuf<uint32_t> perm, prow, pparent;  // units sorted by output row (stable), their rows, parents
-  DevBuf<uint32_t> segs;             // per segment: first, end, piece slot (~0u: whole rows)
-  DevBuf<uint32_t> pieces;           // per long row: row, first piece slot, pieces
-  DevBuf<double> piece_sum;          // per piece: its sum (ldr)
-  uint32_t nsegs = 0, nlong = 0, npieces = 0;
-  DevBuf<float> prefix[2];           // prefix rows of levels 0..out-1 (ping-pong)
+  std::unique_ptr<PullWalk> pull;    // scatter of level `out` as a pull (deterministic)
   bool has_store() const {
     for (int l = 0; l < kMaxModes; ++l)
       if (store[l]) return true;

@@ -2,7 +2,7 @@
 // and BF16 factor rows, packed FP32 products.
 #pragma once
 
-#include "mttkrp.cuh"
+#include "pull.cuh"
 
 namespace adatm {
 
@@ -28,24 +28,6 @@ __device__ __forceinline__ uint64_t pack2(float x, float y) {
 __device__ __forceinline__ void unpack2(uint64_t p, float &x, float &y) {
   asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(p));
 }
-template <int V>
-__device__ __forceinline__ fv<V> fv_mul(const fv<V> &a, const fv<V> &b) {
-  fv<V> r;
-  if constexpr (V == 1) {
-    r.x[0] = a.x[0] * b.x[0];
-  } else {
-#pragma unroll
-    for (int i = 0; i < V; i += 2) {
-      uint64_t t;
-      asm("mul.rn.f32x2 %0, %1, %2;"
-          : "=l"(t)
-          : "l"(pack2(a.x[i], a.x[i + 1])), "l"(pack2(b.x[i], b.x[i + 1])));
-      unpack2(t, r.x[i], r.x[i + 1]);
-    }
-  }
-  return r;
-}
-
 // Columns col..col+V-1 of factor row `row` (FP32 or BF16 storage).
 template <int V, FactorType FT>
 __device__ __forceinline__ fv<V> ld_factor(const void *U, uint32_t row, int ldr, int col, bool act) {
@@ -304,6 +286,11 @@ __device__ __forceinline__ uint32_t ld_stream(const uint8_t *p) {
   uint32_t v;
   asm("ld.global.nc.L2::256B.u8 %0, [%1];" : "=r"(v) : "l"(p));
   return v;
+}
+
+// An FP32 row that is read once: it takes no room in L1.
+__device__ __forceinline__ void ld_row_once(RawRow<4, FactorType::F32> &a, const char *p) {
+  asm("ld.global.nc.L1::no_allocate.v2.b64 {%0, %1}, [%2];" : "=l"(a.r.w[0]), "=l"(a.r.w[1]) : "l"(p));
 }
 
 }  // namespace adatm
