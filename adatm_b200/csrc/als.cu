@@ -10,23 +10,23 @@ namespace {
 void set_attributes();
 }
 
-void AlsWork::init(int nmodes_, int R_, int nblocks_, int max_iters) {
+void AlsWork::init(int nmodes_, int R_, int nblocks_, int max_iters, cudaStream_t s) {
   nmodes = nmodes_;
   R = R_;
   ldr = ldr_of(R_);
   nblocks = nblocks_;
-  vinv64.alloc((size_t)R * R);
-  part_gram.alloc((size_t)nblocks * R * R);
-  part_max.alloc((size_t)nblocks * R);
-  part_inner.alloc((size_t)nblocks * R);
-  lambda.alloc(R);
-  scalars.alloc(8);
-  iter.alloc(1);
+  vinv64.alloc((size_t)R * R, s);
+  part_gram.alloc((size_t)nblocks * R * R, s);
+  part_max.alloc((size_t)nblocks * R, s);
+  part_inner.alloc((size_t)nblocks * R, s);
+  lambda.alloc(R, s);
+  scalars.alloc(8, s);
+  iter.alloc(1, s);
   max_trace = std::max(1, max_iters);
-  fit_trace.alloc(max_trace);
-  ADATM_CUDA(cudaMemset(scalars.get(), 0, 8 * sizeof(double)));
-  ADATM_CUDA(cudaMemset(iter.get(), 0, sizeof(int)));
-  ADATM_CUDA(cudaMemset(fit_trace.get(), 0, max_trace * sizeof(double)));
+  fit_trace.alloc(max_trace, s);
+  ADATM_CUDA(cudaMemsetAsync(scalars.get(), 0, 8 * sizeof(double), s));
+  ADATM_CUDA(cudaMemsetAsync(iter.get(), 0, sizeof(int), s));
+  ADATM_CUDA(cudaMemsetAsync(fit_trace.get(), 0, max_trace * sizeof(double), s));
   set_attributes();
 }
 
@@ -569,7 +569,7 @@ void gram(const float *A, uint64_t rows, int R, int ldr, double *G, AlsWork &w, 
 
 void frob_sq(const double *vals, uint64_t n, AlsWork &w, cudaStream_t s) {
   const int blocks = 256;
-  if (w.frob_part.n < (size_t)blocks) w.frob_part.alloc(blocks);
+  if (w.frob_part.n < (size_t)blocks) w.frob_part.alloc(blocks, s);
   k_frob_partial<<<blocks, kFrobThreads, 0, s>>>(vals, n, w.frob_part.get());
   ADATM_LAUNCH();
   k_frob_final<<<1, 32, 0, s>>>(w.frob_part.get(), blocks, w.scalars.get());

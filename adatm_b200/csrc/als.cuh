@@ -21,7 +21,7 @@ struct AlsWork {
   DevBuf<double> fit_trace;              // per-iteration fits
   DevBuf<double> frob_part;              // partial sums of ||X||^2
   int max_trace = 0;
-  void init(int nmodes_, int R_, int nblocks_, int max_iters);
+  void init(int nmodes_, int R_, int nblocks_, int max_iters, cudaStream_t s);
 };
 
 struct GramSet {

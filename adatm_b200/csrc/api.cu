@@ -62,9 +62,11 @@ cudaStream_t new_stream() {
 
 struct StreamOwner {
   cudaStream_t s = nullptr;
-  StreamOwner() : s(new_stream()) {}
+  StreamOwner() : s(new_stream()) { stream_opened(s); }
   ~StreamOwner() {
-    if (s) cudaStreamDestroy(s);
+    if (!s) return;
+    stream_closed(s);
+    cudaStreamDestroy(s);
   }
 };
 
@@ -1494,7 +1496,7 @@ int adatm_gram(const float *A, uint64_t rows, int R, int ldr, double *G) {
     ADATM_CUDA(cudaGetDevice(&dev));
     ADATM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     AlsWork w;
-    w.init(1, R, 2 * sms, 1);
+    w.init(1, R, 2 * sms, 1, s.s);
     w.ldr = ldr;
     gram(A, rows, R, ldr, G, w, s.s);
     ADATM_CUDA(cudaStreamSynchronize(s.s));

@@ -273,16 +273,16 @@ struct SortBufs {
 // b.keys/b.order.
 template <int W>
 void sort_keys(const IdxPtrs &ip, uint64_t n, const KeySpec &spec, SortBufs<W> &b, cudaStream_t s) {
-  b.k0.alloc(n);
-  b.k1.alloc(n);
-  b.o0.alloc(n);
-  b.o1.alloc(n);
+  b.k0.alloc(n, s);
+  b.k1.alloc(n, s);
+  b.o0.alloc(n, s);
+  b.o1.alloc(n, s);
   const unsigned blocks = (unsigned)((n + 255) / 256);
   k_pack<W><<<blocks, 256, 0, s>>>(ip, spec, n, b.k0.get(), b.o0.get());
   ADATM_LAUNCH();
   const uint32_t ntiles = (uint32_t)((n + RsTile<W>::tile - 1) / RsTile<W>::tile);
-  DevBuf<uint32_t> counts((size_t)256 * ntiles), offs((size_t)256 * ntiles),
-      tmp(scan_tmp_words((size_t)256 * ntiles));
+  DevBuf<uint32_t> counts((size_t)256 * ntiles, s), offs((size_t)256 * ntiles, s),
+      tmp(scan_tmp_words((size_t)256 * ntiles), s);
   ADATM_CUDA(cudaFuncSetAttribute(k_rs_scatter<W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)RsTile<W>::smem));
   Key<W> *kin = b.k0.get(), *kout = b.k1.get();
@@ -467,8 +467,8 @@ void count_levels(const SortBufs<W> &b, uint64_t n, const KeySpec &spec, DevBuf<
                   uint32_t &ntiles, uint64_t *nfibs, cudaStream_t s) {
   const int nl = spec.nlev - 1;
   ntiles = (uint32_t)((n + kLvTile - 1) / kLvTile);
-  DevBuf<uint32_t> counts((size_t)nl * ntiles), tmp(scan_tmp_words(ntiles)), totals(kMaxModes);
-  offs.alloc((size_t)nl * ntiles);
+  DevBuf<uint32_t> counts((size_t)nl * ntiles, s), tmp(scan_tmp_words(ntiles), s), totals(kMaxModes, s);
+  offs.alloc((size_t)nl * ntiles, s);
   k_level_count<W><<<ntiles, kLvThreads, 0, s>>>(b.keys, n, spec, counts.get(), ntiles);
   ADATM_LAUNCH();
   for (int l = 0; l < nl; ++l)
@@ -497,7 +497,7 @@ void build_close_depths(DevCsf &out, cudaStream_t s) {
   const int N = out.nmodes;
   for (int l = 1; l < N; ++l) {
     const uint64_t n = l == N - 1 ? out.nnz : out.nfibs[l];
-    out.cdepth[l].alloc(n);
+    out.cdepth[l].alloc(n, s);
     if (n == 0) continue;
     ADATM_CUDA(cudaMemsetAsync(out.cdepth[l].get(), 0, n, s));
     const uint64_t np = out.nfibs[l - 1];
@@ -524,20 +524,20 @@ void build_w(const DevCoo &coo, const uint64_t *perm, const KeySpec &spec, DevCs
     lo.fids[l] = nullptr;
   }
   for (int l = 0; l < N - 1; ++l) {
-    out.fptr[l].alloc(out.nfibs[l] + 1);
-    out.fids[l].alloc(out.nfibs[l]);
+    out.fptr[l].alloc(out.nfibs[l] + 1, s);
+    out.fids[l].alloc(out.nfibs[l], s);
     lo.fptr[l] = out.fptr[l].get();
     lo.fids[l] = out.fids[l].get();
   }
-  out.fids[N - 1].alloc(n);
+  out.fids[N - 1].alloc(n, s);
   lo.fids[N - 1] = out.fids[N - 1].get();
-  out.vals64.alloc(n);
-  out.vals32.alloc(n);
+  out.vals64.alloc(n, s);
+  out.vals32.alloc(n, s);
   k_level_fill<W><<<ntiles, kLvThreads, 0, s>>>(b.keys, b.order, n, spec, offs.get(), ntiles, lo,
                                                 coo.vals.get(), out.vals64.get(),
                                                 out.vals32.get());
   ADATM_LAUNCH();
-  DevBuf<uint32_t> totals(kMaxModes);
+  DevBuf<uint32_t> totals(kMaxModes, s);
   uint32_t ht[kMaxModes] = {0};
   for (int l = 0; l < N - 1; ++l) ht[l] = (uint32_t)out.nfibs[l];
   ADATM_CUDA(cudaMemcpyAsync(totals.get(), ht, sizeof(ht), cudaMemcpyHostToDevice, s));
@@ -617,7 +617,7 @@ void clean_w(const DevCoo &in, DevCoo &out, const KeySpec &spec, cudaStream_t s)
   for (int m = 0; m < N; ++m) perm[m] = (uint64_t)m;
   SortBufs<W> b;
   sort_keys<W>(in, perm, spec, b, s);
-  DevBuf<uint32_t> flags(n), seg(n), tmp(scan_tmp_words(n));
+  DevBuf<uint32_t> flags(n, s), seg(n, s), tmp(scan_tmp_words(n), s);
   const unsigned blocks = (unsigned)((n + 255) / 256);
   k_newkey_flags<W><<<blocks, 256, 0, s>>>(b.keys, n, flags.get());
   ADATM_LAUNCH();
@@ -642,7 +642,7 @@ void clean_w(const DevCoo &in, DevCoo &out, const KeySpec &spec, cudaStream_t s)
   // compact empty slices of every mode
   for (int m = 0; m < N; ++m) {
     const uint64_t d = in.dims[m];
-    DevBuf<uint32_t> used(d), map(d), mtmp(scan_tmp_words(d));
+    DevBuf<uint32_t> used(d, s), map(d, s), mtmp(scan_tmp_words(d), s);
     ADATM_CUDA(cudaMemsetAsync(used.get(), 0, d * sizeof(uint32_t), s));
     const unsigned ub = (unsigned)((nu + 255) / 256);
     k_mark_used<<<ub, 256, 0, s>>>(out.idx[m].get(), nu, used.get());
@@ -726,8 +726,8 @@ void coo_upload(DevCoo &out, int nmodes, uint64_t nnz, const uint64_t *dims,
   if (nnz >= 0xFFFFFFFFull) throw BadInput("nnz must be below 2^32-1");
   out.nmodes = nmodes;
   out.nnz = nnz;
-  DevBuf<uint64_t> tmp(nnz);
-  DevBuf<unsigned int> bad(1);
+  DevBuf<uint64_t> tmp(nnz, s);
+  DevBuf<unsigned int> bad(1, s);
   ADATM_CUDA(cudaMemsetAsync(bad.get(), 0, sizeof(unsigned int), s));
   for (int m = 0; m < nmodes; ++m) {
     if (dims[m] == 0 || dims[m] >= 0xFFFFFFFFull) throw BadInput("dimension out of range");
@@ -803,7 +803,7 @@ void coo_generate(DevCoo &out, int nmodes, const uint64_t *dims, uint64_t nnz,
       }
       for (uint64_t k = 0; k < dims[m]; ++k) c[k] /= acc;
       c[dims[m] - 1] = 1.0;
-      cdfs[m].alloc(dims[m]);
+      cdfs[m].alloc(dims[m], s);
       ADATM_CUDA(cudaMemcpyAsync(cdfs[m].get(), c.data(), dims[m] * sizeof(double),
                                  cudaMemcpyHostToDevice, s));
       a.cdf[m] = cdfs[m].get();
@@ -829,7 +829,7 @@ void csf_build(const DevCoo &coo, const uint64_t *perm, DevCsf &out, cudaStream_
   if (coo.nnz == 0) {
     for (int l = 0; l < N - 1; ++l) {
       out.nfibs[l] = 0;
-      out.fptr[l].alloc(1);
+      out.fptr[l].alloc(1, s);
       ADATM_CUDA(cudaMemsetAsync(out.fptr[l].get(), 0, sizeof(uint32_t), s));
     }
     out.nfibs[N - 1] = 0;
@@ -867,7 +867,7 @@ void sort_by_row(const uint32_t *row, uint64_t n, uint64_t nrows, DevBuf<uint32_
   ip.p[0] = row;
   SortBufs<1> b;
   sort_keys<1>(ip, n, spec, b, s);
-  sorted.alloc(n);
+  sorted.alloc(n, s);
   k_narrow_keys<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(b.keys, n, sorted.get());
   ADATM_LAUNCH();
   ADATM_CUDA(cudaStreamSynchronize(s));
@@ -880,7 +880,7 @@ void csf_download(const DevCsf &c, HostCsfArrays &h, cudaStream_t s) {
   h.fids.assign(N, {});
   uint64_t maxn = 1;
   for (int l = 0; l < N; ++l) maxn = std::max<uint64_t>(maxn, c.nfibs[l] + 1);
-  DevBuf<uint64_t> wide(maxn);
+  DevBuf<uint64_t> wide(maxn, s);
   auto pull = [&](const DevBuf<uint32_t> &src, uint64_t n, std::vector<uint64_t> &dst) {
     dst.assign(n, 0);
     if (n == 0 || src.get() == nullptr) return;

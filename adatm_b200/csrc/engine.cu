@@ -109,7 +109,7 @@ Engine::Engine(std::shared_ptr<const DevCoo> coo, std::vector<std::shared_ptr<De
     for (uint64_t deg = 0; deg < gp.n_imten; ++deg) {
       const uint64_t lvl = gp.begin_imten - 1 - deg;
       const size_t n = (size_t)csf_[g]->nfibs[lvl] * ldr_;
-      memo_[g][deg].alloc(n);
+      memo_[g][deg].alloc(n, stream_);
       ADATM_CUDA(cudaMemsetAsync(memo_[g][deg].get(), 0, n * sizeof(float), stream_));
     }
   }
@@ -120,10 +120,10 @@ Engine::Engine(std::shared_ptr<const DevCoo> coo, std::vector<std::shared_ptr<De
     maxdim = std::max(maxdim, coo_->dims[m]);
     rows += coo_->dims[m];
   }
-  factors_.alloc((size_t)rows * ldr_);
+  factors_.alloc((size_t)rows * ldr_, stream_);
   ADATM_CUDA(cudaMemsetAsync(factors_.get(), 0, factors_.bytes(), stream_));
   if (opt_.factor_type == FactorType::BF16) {
-    factors16_.alloc((size_t)rows * ldr_);
+    factors16_.alloc((size_t)rows * ldr_, stream_);
     ADATM_CUDA(cudaMemsetAsync(factors16_.get(), 0, factors16_.bytes(), stream_));
   }
   rows = 0;
@@ -131,16 +131,16 @@ Engine::Engine(std::shared_ptr<const DevCoo> coo, std::vector<std::shared_ptr<De
     A_[m] = factors_.get() + (size_t)rows * ldr_;
     Ab_[m] = factors16_.get() ? factors16_.get() + (size_t)rows * ldr_ : nullptr;
     rows += coo_->dims[m];
-    G_[m].alloc((size_t)R_ * R_);
+    G_[m].alloc((size_t)R_ * R_, stream_);
   }
-  M_.alloc((size_t)maxdim * ldr_);
+  M_.alloc((size_t)maxdim * ldr_, stream_);
   int sms = 148;
   {
     int dev = 0;
     ADATM_CUDA(cudaGetDevice(&dev));
     ADATM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   }
-  w_.init(N, (int)R_, 2 * sms, opt_.max_iters);
+  w_.init(N, (int)R_, 2 * sms, opt_.max_iters, stream_);
   ADATM_CUDA(cudaStreamCreateWithFlags(&side_, cudaStreamNonBlocking));
   ADATM_CUDA(cudaEventCreateWithFlags(&fork_, cudaEventDisableTiming));
   ADATM_CUDA(cudaEventCreateWithFlags(&join_, cudaEventDisableTiming));
@@ -158,6 +158,9 @@ Engine::~Engine() {
   if (join_) cudaEventDestroy(join_);
   if (fork_) cudaEventDestroy(fork_);
   if (staged_) cudaEventDestroy(staged_);
+  // the buffers go back for later work on the engine's stream: the other
+  // streams' work on them ends first
+  if (side_) cudaStreamSynchronize(side_);
   if (copy_) cudaStreamSynchronize(copy_);
   for (auto ev : updated_)
     if (ev) cudaEventDestroy(ev);

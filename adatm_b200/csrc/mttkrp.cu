@@ -882,7 +882,7 @@ void prepare_spans(TreeWalk &w, cudaStream_t s) {
   if (d > 0) {
     // the level-d sums are stored, then pulled (or, with atomics, scattered)
     // into the output rows
-    w.level_rows.alloc((size_t)std::max<uint64_t>(c.nfibs[d], 1) * w.ldr);
+    w.level_rows.alloc((size_t)std::max<uint64_t>(c.nfibs[d], 1) * w.ldr, s);
     ADATM_CUDA(cudaMemsetAsync(w.level_rows.get(), 0, w.level_rows.bytes(), s));
     w.store[d] = w.level_rows.get();
     if (!w.deterministic) {
@@ -902,9 +902,9 @@ void prepare_spans(TreeWalk &w, cudaStream_t s) {
   for (int l = 0; l < S; ++l)
     if (w.store[l] != nullptr || (l == 0 && d == 0)) w.span_lev[l] = w.span_nlev++;
   if (w.nchunks == 0 || w.span_nlev == 0) return;
-  w.span.alloc((size_t)w.nchunks * w.span_nlev * 2 * w.ldr);
+  w.span.alloc((size_t)w.nchunks * w.span_nlev * 2 * w.ldr, s);
   ADATM_CUDA(cudaMemsetAsync(w.span.get(), 0, w.span.bytes(), s));  // padding columns stay zero
-  DevBuf<uint32_t> cut((size_t)w.span_nlev * w.nchunks);
+  DevBuf<uint32_t> cut((size_t)w.span_nlev * w.nchunks, s);
   k_cut_nodes<<<(w.nchunks + 255) / 256, 256, 0, s>>>(make_args(w, nullptr, nullptr), cut.get());
   ADATM_LAUNCH();
   int level_of[kMaxModes];
@@ -932,7 +932,7 @@ void find_hot_rows(TreeWalk &w, cudaStream_t s) {
   // rows than kHotScanRows keep the plain scatter
   if (rows64 == 0 || rows64 > kHotScanRows) return;
   const uint32_t rows = (uint32_t)rows64;
-  DevBuf<uint32_t> count(rows);
+  DevBuf<uint32_t> count(rows, s);
   ADATM_CUDA(cudaMemsetAsync(count.get(), 0, rows * sizeof(uint32_t), s));
   const unsigned blocks = (unsigned)std::min<uint64_t>((w.nunits + 255) / 256, 4096);
   k_row_count<<<blocks, 256, 0, s>>>(c.fids[w.out].get(), w.nunits, rows, count.get());
@@ -951,8 +951,8 @@ void find_hot_rows(TreeWalk &w, cudaStream_t s) {
   if (hot.empty()) return;
   std::vector<uint8_t> slot(rows, 0xFF);
   for (size_t i = 0; i < hot.size(); ++i) slot[hot[i]] = (uint8_t)i;
-  w.hot_slot.alloc(rows);
-  w.hot_rows.alloc(hot.size());
+  w.hot_slot.alloc(rows, s);
+  w.hot_rows.alloc(hot.size(), s);
   ADATM_CUDA(cudaMemcpyAsync(w.hot_slot.get(), slot.data(), rows, cudaMemcpyHostToDevice, s));
   ADATM_CUDA(cudaMemcpyAsync(w.hot_rows.get(), hot.data(), hot.size() * sizeof(uint32_t),
                              cudaMemcpyHostToDevice, s));
@@ -987,7 +987,7 @@ void walk_prepare(TreeWalk &w, cudaStream_t s) {
   if (w.chunk == 0) w.chunk = auto_chunk(w);
   w.chunk = std::min(w.chunk, 1u << 30);  // offsets in a chunk are 32-bit numbers
   w.nchunks = (uint32_t)((w.nunits + w.chunk - 1) / w.chunk);
-  w.sched.alloc((size_t)std::max<uint32_t>(w.nchunks, 1) * (w.src + 1) + 1);  // + the chunk counter
+  w.sched.alloc((size_t)std::max<uint32_t>(w.nchunks, 1) * (w.src + 1) + 1, s);  // + the chunk counter
   w.nhot = 0;
   w.hot_slot.reset();
   w.hot_rows.reset();

@@ -257,20 +257,19 @@ void pull_prepare(PullWalk &p, const DevCsf &c, int d, bool leaf, int R, int ldr
   DevBuf<uint32_t> parent[kMaxModes];
   for (int l = 1; l <= d; ++l) {
     const uint64_t n = c.nfibs[l];
-    DevBuf<uint32_t> flags(n), tmp(scan_tmp_words(n));
-    parent[l].alloc(n);
+    DevBuf<uint32_t> flags(n, s), tmp(scan_tmp_words(n), s);
+    parent[l].alloc(n, s);
     k_last_child<<<blocks_of(n), 256, 0, s>>>(c.cdepth[l].get(), n, flags.get());
     ADATM_LAUNCH();
     exclusive_scan_u32(flags.get(), parent[l].get(), n, tmp.get(), s);
-    ADATM_CUDA(cudaStreamSynchronize(s));
     a.parent[l] = parent[l].get();
   }
   for (int l = 0; l < d; ++l) {
-    p.anc[l].alloc(p.n);
+    p.anc[l].alloc(p.n, s);
     a.anc[l] = p.anc[l].get();
     a.fids[l] = c.fids[l].get();
   }
-  if (leaf) p.vals.alloc(p.n);
+  if (leaf) p.vals.alloc(p.n, s);
   k_ancestors<<<blocks_of(p.n), 256, 0, s>>>(p.perm.get(), p.n, a, c.vals32.get(), leaf ? p.vals.get() : nullptr);
   ADATM_LAUNCH();
   // segments: one per walker slot of a full device while that is at most 128
@@ -279,9 +278,9 @@ void pull_prepare(PullWalk &p, const DevCsf &c, int d, bool leaf, int R, int ldr
   const uint64_t u = per_slot <= 128 ? per_slot : std::min<uint64_t>(128, per_slot / 4);
   p.seg = (uint32_t)std::max<uint64_t>(16, (u + 15) / 16 * 16);
   p.nsegs = (uint32_t)((p.n + p.seg - 1) / p.seg);
-  p.span.alloc((size_t)p.nsegs * 2 * ldr);
+  p.span.alloc((size_t)p.nsegs * 2 * ldr, s);
   ADATM_CUDA(cudaMemsetAsync(p.span.get(), 0, p.span.bytes(), s));  // padding columns stay zero
-  DevBuf<uint32_t> cut(p.nsegs);
+  DevBuf<uint32_t> cut(p.nsegs, s);
   k_cut_rows<<<blocks_of(p.nsegs), 256, 0, s>>>(p.row.get(), p.seg, p.nsegs, cut.get());
   ADATM_LAUNCH();
   const int level = 0;

@@ -224,7 +224,7 @@ void span_prepare(SpanSums &s, const uint32_t *cut, int nlev, const int *level_o
   a.nlev = nlev;
   a.nch = nch;
   for (int k = 0; k < kMaxModes; ++k) a.level_of[k] = k < nlev ? level_of[k] : 0;
-  DevBuf<uint32_t> flags(2 * n), at(2 * n), tmp(scan_tmp_words(n));
+  DevBuf<uint32_t> flags(2 * n, stream), at(2 * n, stream), tmp(scan_tmp_words(n), stream);
   uint32_t *begin = flags.get(), *end = begin + n, *ib = at.get(), *ie = ib + n;
   k_chain_flags<<<blocks_of(n), 256, 0, stream>>>(cut, a, begin, end);
   ADATM_LAUNCH();
@@ -232,10 +232,11 @@ void span_prepare(SpanSums &s, const uint32_t *cut, int nlev, const int *level_o
   exclusive_scan_u32(end, ie, n, tmp.get(), stream);
   const uint32_t nc = total_of(begin, ib, n, stream);
   if (nc == 0) return;
-  s.chain.alloc((size_t)nc * kChainWords);
+  s.chain.alloc((size_t)nc * kChainWords, stream);
   k_chain_bounds<<<blocks_of(n), 256, 0, stream>>>(cut, a, begin, ib, end, ie, s.chain.get());
   ADATM_LAUNCH();
-  DevBuf<uint32_t> sizes(2 * (size_t)nc), first(2 * (size_t)nc), tmp2(scan_tmp_words(nc));
+  DevBuf<uint32_t> sizes(2 * (size_t)nc, stream), first(2 * (size_t)nc, stream),
+      tmp2(scan_tmp_words(nc), stream);
   uint32_t *ng = sizes.get(), *nm = ng + nc, *g0 = first.get(), *m0 = g0 + nc;
   k_chain_sizes<<<blocks_of(nc), 256, 0, stream>>>(s.chain.get(), nc, ng, nm);
   ADATM_LAUNCH();
@@ -244,13 +245,13 @@ void span_prepare(SpanSums &s, const uint32_t *cut, int nlev, const int *level_o
   s.ngroups = total_of(ng, g0, nc, stream);
   s.nmids = total_of(nm, m0, nc, stream);
   s.nchains = nc;
-  s.group_chain.alloc(s.ngroups);
+  s.group_chain.alloc(s.ngroups, stream);
   k_chain_groups_of<<<blocks_of((uint64_t)nc * 32), 256, 0, stream>>>(s.chain.get(), nc, g0, m0,
                                                                       s.group_chain.get());
   ADATM_LAUNCH();
-  s.gsum.alloc((size_t)s.ngroups * ldr);
-  s.msum.alloc((size_t)s.nmids * ldr);
-  s.arrived.alloc((size_t)s.nmids + nc);
+  s.gsum.alloc((size_t)s.ngroups * ldr, stream);
+  s.msum.alloc((size_t)s.nmids * ldr, stream);
+  s.arrived.alloc((size_t)s.nmids + nc, stream);
   ADATM_CUDA(cudaMemsetAsync(s.arrived.get(), 0, s.arrived.bytes(), stream));
   ADATM_CUDA(cudaStreamSynchronize(stream));  // the scratch above is given back here
 }
