@@ -870,7 +870,6 @@ void sort_by_row(const uint32_t *row, uint64_t n, uint64_t nrows, DevBuf<uint32_
   sorted.alloc(n, s);
   k_narrow_keys<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(b.keys, n, sorted.get());
   ADATM_LAUNCH();
-  ADATM_CUDA(cudaStreamSynchronize(s));
   perm = std::move(b.order == b.o0.get() ? b.o0 : b.o1);
 }
 

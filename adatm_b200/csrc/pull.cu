@@ -285,7 +285,6 @@ void pull_prepare(PullWalk &p, const DevCsf &c, int d, bool leaf, int R, int ldr
   ADATM_LAUNCH();
   const int level = 0;
   span_prepare(p.sums, cut.get(), 1, &level, p.nsegs, ldr, s);
-  ADATM_CUDA(cudaStreamSynchronize(s));
   if (leaf) p.perm.reset();
 }
 

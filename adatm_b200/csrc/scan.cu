@@ -101,6 +101,31 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_final(const uint32_t *in,
   }
 }
 
+// One block for short arrays: one launch in the place of three.
+__global__ void __launch_bounds__(kScanThreads) k_scan_short(const uint32_t *in, uint32_t *out, size_t n) {
+  __shared__ uint32_t tot;
+  uint32_t carry = 0;
+  for (size_t base = 0; base < n; base += kScanTile) {
+    uint32_t v[kScanItems];
+    uint32_t s = 0;
+#pragma unroll
+    for (int i = 0; i < kScanItems; ++i) {
+      const size_t idx = base + (size_t)threadIdx.x * kScanItems + i;
+      v[i] = idx < n ? in[idx] : 0;
+      s += v[i];
+    }
+    uint32_t ex = block_excl_scan(s, &tot) + carry;
+#pragma unroll
+    for (int i = 0; i < kScanItems; ++i) {
+      const size_t idx = base + (size_t)threadIdx.x * kScanItems + i;
+      if (idx < n) out[idx] = ex;
+      ex += v[i];
+    }
+    carry += tot;
+    __syncthreads();
+  }
+}
+
 }  // namespace
 
 size_t scan_tmp_words(size_t n) { return (n + kScanTile - 1) / kScanTile + 1; }
@@ -108,6 +133,11 @@ size_t scan_tmp_words(size_t n) { return (n + kScanTile - 1) / kScanTile + 1; }
 void exclusive_scan_u32(const uint32_t *in, uint32_t *out, size_t n, uint32_t *tmp,
                         cudaStream_t stream) {
   if (n == 0) return;
+  if (n <= 4 * (size_t)kScanTile) {  // four rounds of one block: about the time of one more launch
+    k_scan_short<<<1, kScanThreads, 0, stream>>>(in, out, n);
+    ADATM_LAUNCH();
+    return;
+  }
   const size_t tiles = (n + kScanTile - 1) / kScanTile;
   k_scan_reduce<<<(unsigned)tiles, kScanThreads, 0, stream>>>(in, n, tmp);
   ADATM_LAUNCH();

@@ -30,34 +30,35 @@ __global__ void k_chain_flags(const uint32_t *cut, CutArgs a, uint32_t *begin, u
 }
 
 // The k-th beginning and the k-th end belong to chain k.
-__global__ void k_chain_bounds(const uint32_t *cut, CutArgs a, const uint32_t *begin, const uint32_t *ib,
-                               const uint32_t *end, const uint32_t *ie, uint32_t *chain) {
+__global__ void k_chain_bounds(const uint32_t *cut, CutArgs a, const uint32_t *begin, const uint32_t *end,
+                               const uint32_t *at, uint32_t nchains, uint32_t *chain) {
   const uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= (uint64_t)a.nlev * a.nch) return;
   const uint32_t c = (uint32_t)(e % a.nch), k = (uint32_t)(e / a.nch);
   if (begin[e]) {
-    uint32_t *o = chain + (size_t)ib[e] * kChainWords;
+    uint32_t *o = chain + (size_t)at[e] * kChainWords;
     o[0] = (uint32_t)a.level_of[k];
     o[1] = cut[e] - 1u;
     o[2] = k;
     o[3] = c;
   }
-  if (end[e]) chain[(size_t)ie[e] * kChainWords + 4] = c;
+  if (end[e]) chain[(size_t)(at[(uint64_t)a.nlev * a.nch + e] - nchains) * kChainWords + 4] = c;
 }
 
-__global__ void k_chain_sizes(uint32_t *chain, uint32_t n, uint32_t *ngroups, uint32_t *nmids) {
+__global__ void k_chain_sizes(uint32_t *chain, uint32_t n, uint32_t *sizes) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0u) sizes[2 * (size_t)n] = 0u;
   if (i >= n) return;
   uint32_t *o = chain + (size_t)i * kChainWords;
   const uint32_t npart = o[4] - o[3] + 2u, ng = (npart + kGroup - 1) / kGroup;
   o[4] = npart;
-  ngroups[i] = ng;
-  o[7] = nmids[i] = ng > kMid ? (ng + kMid - 1) / kMid : 0u;
+  sizes[i] = ng;
+  o[7] = sizes[(size_t)n + i] = ng > kMid ? (ng + kMid - 1) / kMid : 0u;
 }
 
 // One warp per chain: its first group and group of groups, and the chain of
 // its groups.
-__global__ void k_chain_groups_of(uint32_t *chain, uint32_t n, const uint32_t *g0, const uint32_t *m0,
+__global__ void k_chain_groups_of(uint32_t *chain, uint32_t n, const uint32_t *first, uint32_t ngroups,
                                   uint32_t *group_chain) {
   const uint32_t i = (uint32_t)(((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
@@ -65,10 +66,10 @@ __global__ void k_chain_groups_of(uint32_t *chain, uint32_t n, const uint32_t *g
   uint32_t *o = chain + (size_t)i * kChainWords;
   const uint32_t ng = (o[4] + kGroup - 1) / kGroup;
   if (lane == 0) {
-    o[5] = g0[i];
-    o[6] = m0[i];
+    o[5] = first[i];
+    o[6] = first[(size_t)n + i] - ngroups;
   }
-  for (uint32_t g = lane; g < ng; g += 32) group_chain[g0[i] + g] = i;
+  for (uint32_t g = lane; g < ng; g += 32) group_chain[first[i] + g] = i;
 }
 
 template <typename T>
@@ -204,13 +205,11 @@ __global__ void __launch_bounds__(128) k_span_sums(const __grid_constant__ SumAr
 
 unsigned blocks_of(uint64_t n) { return (unsigned)((n + 255) / 256); }
 
-// The last value of an exclusive scan plus the last value scanned.
-uint32_t total_of(const uint32_t *in, const uint32_t *scan, uint64_t n, cudaStream_t s) {
-  uint32_t a = 0, b = 0;
-  ADATM_CUDA(cudaMemcpyAsync(&a, in + n - 1, sizeof(a), cudaMemcpyDeviceToHost, s));
-  ADATM_CUDA(cudaMemcpyAsync(&b, scan + n - 1, sizeof(b), cudaMemcpyDeviceToHost, s));
+uint32_t to_host(const uint32_t *p, cudaStream_t s) {
+  uint32_t v = 0;
+  ADATM_CUDA(cudaMemcpyAsync(&v, p, sizeof(v), cudaMemcpyDeviceToHost, s));
   ADATM_CUDA(cudaStreamSynchronize(s));
-  return a + b;
+  return v;
 }
 
 }  // namespace
@@ -224,36 +223,37 @@ void span_prepare(SpanSums &s, const uint32_t *cut, int nlev, const int *level_o
   a.nlev = nlev;
   a.nch = nch;
   for (int k = 0; k < kMaxModes; ++k) a.level_of[k] = k < nlev ? level_of[k] : 0;
-  DevBuf<uint32_t> flags(2 * n, stream), at(2 * n, stream), tmp(scan_tmp_words(n), stream);
-  uint32_t *begin = flags.get(), *end = begin + n, *ib = at.get(), *ie = ib + n;
+  // flags of the beginnings, then of the ends, in one scan: the chain that
+  // ends at a boundary is the number of ends before it
+  DevBuf<uint32_t> flags(2 * n, stream), at(2 * n, stream), tmp(scan_tmp_words(2 * n), stream);
+  uint32_t *begin = flags.get(), *end = begin + n;
   k_chain_flags<<<blocks_of(n), 256, 0, stream>>>(cut, a, begin, end);
   ADATM_LAUNCH();
-  exclusive_scan_u32(begin, ib, n, tmp.get(), stream);
-  exclusive_scan_u32(end, ie, n, tmp.get(), stream);
-  const uint32_t nc = total_of(begin, ib, n, stream);
+  exclusive_scan_u32(begin, at.get(), 2 * n, tmp.get(), stream);
+  const uint32_t nc = to_host(at.get() + n, stream);
   if (nc == 0) return;
   s.chain.alloc((size_t)nc * kChainWords, stream);
-  k_chain_bounds<<<blocks_of(n), 256, 0, stream>>>(cut, a, begin, ib, end, ie, s.chain.get());
+  k_chain_bounds<<<blocks_of(n), 256, 0, stream>>>(cut, a, begin, end, at.get(), nc, s.chain.get());
   ADATM_LAUNCH();
-  DevBuf<uint32_t> sizes(2 * (size_t)nc, stream), first(2 * (size_t)nc, stream),
-      tmp2(scan_tmp_words(nc), stream);
-  uint32_t *ng = sizes.get(), *nm = ng + nc, *g0 = first.get(), *m0 = g0 + nc;
-  k_chain_sizes<<<blocks_of(nc), 256, 0, stream>>>(s.chain.get(), nc, ng, nm);
+  // groups, then groups of groups, of every chain, and a last 0
+  DevBuf<uint32_t> sizes(2 * (size_t)nc + 1, stream), first(2 * (size_t)nc + 1, stream),
+      tmp2(scan_tmp_words(2 * (size_t)nc + 1), stream);
+  k_chain_sizes<<<blocks_of(nc), 256, 0, stream>>>(s.chain.get(), nc, sizes.get());
   ADATM_LAUNCH();
-  exclusive_scan_u32(ng, g0, nc, tmp2.get(), stream);
-  exclusive_scan_u32(nm, m0, nc, tmp2.get(), stream);
-  s.ngroups = total_of(ng, g0, nc, stream);
-  s.nmids = total_of(nm, m0, nc, stream);
+  exclusive_scan_u32(sizes.get(), first.get(), 2 * (size_t)nc + 1, tmp2.get(), stream);
+  ADATM_CUDA(cudaMemcpyAsync(&s.nmids, first.get() + 2 * (size_t)nc, sizeof(uint32_t), cudaMemcpyDeviceToHost,
+                             stream));
+  s.ngroups = to_host(first.get() + nc, stream);
+  s.nmids -= s.ngroups;
   s.nchains = nc;
   s.group_chain.alloc(s.ngroups, stream);
-  k_chain_groups_of<<<blocks_of((uint64_t)nc * 32), 256, 0, stream>>>(s.chain.get(), nc, g0, m0,
+  k_chain_groups_of<<<blocks_of((uint64_t)nc * 32), 256, 0, stream>>>(s.chain.get(), nc, first.get(), s.ngroups,
                                                                       s.group_chain.get());
   ADATM_LAUNCH();
   s.gsum.alloc((size_t)s.ngroups * ldr, stream);
   s.msum.alloc((size_t)s.nmids * ldr, stream);
   s.arrived.alloc((size_t)s.nmids + nc, stream);
   ADATM_CUDA(cudaMemsetAsync(s.arrived.get(), 0, s.arrived.bytes(), stream));
-  ADATM_CUDA(cudaStreamSynchronize(stream));  // the scratch above is given back here
 }
 
 template <typename T>
