@@ -477,7 +477,7 @@ void Engine::mttkrp_with(int mode, int tree, int tag, double *out) {
     if (!slot) slot = make_walk(mode, tree, tag);
     w = slot.get();
   }
-  ADATM_CUDA(cudaMemsetAsync(out, 0, (size_t)coo_->dims[mode] * ldr_ * sizeof(double), stream_));
+  clear_output(*w, mode, out);
   walk_launch(*w, level_factors(tree, opt_.factor_type), opt_.factor_type, out, stream_);
 }
 
@@ -491,8 +491,13 @@ LevelFactors Engine::level_factors(int g, FactorType ft) const {
   return f;
 }
 
+void Engine::clear_output(const TreeWalk &w, int mode, double *out) {
+  if (!walk_fills_output(w))
+    ADATM_CUDA(cudaMemsetAsync(out, 0, (size_t)coo_->dims[mode] * ldr_ * sizeof(double), stream_));
+}
+
 void Engine::mttkrp_as(int mode, double *out, FactorType ft) {
-  ADATM_CUDA(cudaMemsetAsync(out, 0, (size_t)coo_->dims[mode] * ldr_ * sizeof(double), stream_));
+  clear_output(*walk_[mode], mode, out);
   walk_launch(*walk_[mode], level_factors((int)plan_.use_csfs[mode], ft), ft, out, stream_);
 }
 
@@ -508,8 +513,8 @@ FactorType Engine::sweep_type(int mode) const {
 }
 
 void Engine::mttkrp_direct(int mode, double *out) {
-  ADATM_CUDA(cudaMemsetAsync(out, 0, (size_t)coo_->dims[mode] * ldr_ * sizeof(double), stream_));
   if (!direct_[mode]) direct_[mode] = make_walk(mode, (int)plan_.use_csfs[mode], 2);
+  clear_output(*direct_[mode], mode, out);
   walk_launch(*direct_[mode], level_factors((int)plan_.use_csfs[mode], opt_.factor_type),
               opt_.factor_type, out, stream_);
 }

@@ -165,6 +165,7 @@ class Engine {
   void build_walks();
   std::unique_ptr<TreeWalk> make_walk(int mode, int tree, int tag);
   LevelFactors level_factors(int g, FactorType ft) const;
+  void clear_output(const TreeWalk &w, int mode, double *out);
 
   std::shared_ptr<const DevCoo> coo_;
   uint64_t R_;

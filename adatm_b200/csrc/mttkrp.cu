@@ -1037,6 +1037,14 @@ void walk_launch(const TreeWalk &w, const LevelFactors &f, FactorType ft, double
   }
 }
 
+bool walk_fills_output(const TreeWalk &w) {
+  if (w.nchunks == 0) return false;
+  if (w.pull) return w.pull->every_row;
+  if (w.src == w.out || w.out > 0) return false;
+  const int vw = walker_cols(w.R, w.walkers > 0 ? w.walkers : default_walkers(w.R));
+  return w.csf->nfibs[0] == w.csf->dims[w.csf->dim_perm[0]] && (w.R % 4 == 0 || vw == 4);
+}
+
 int walk_kernels(const TreeWalk &w) {
   if (w.nchunks == 0) return 0;
   int k = 0;

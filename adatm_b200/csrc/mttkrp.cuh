@@ -95,8 +95,13 @@ bool walkers_supported(int R, int W);
 // unit, plus a bit mask of the levels whose node began before the chunk.
 void walk_prepare(TreeWalk &w, cudaStream_t s);
 
+// Whether the walk writes every value of its output rows, so that they need
+// no clearing: every row has units, nothing is added with atomics, and the
+// padding columns are written.
+bool walk_fills_output(const TreeWalk &w);
+
 // Launch the walk: output rows (FP64, dims x ldr) must be zero beforehand
-// (the caller clears them).
+// unless the walk fills them (the caller clears them).
 void walk_launch(const TreeWalk &w, const LevelFactors &f, FactorType ft, double *out,
                  cudaStream_t s);
 

@@ -205,6 +205,13 @@ __global__ void k_ancestors(const uint32_t *perm, uint64_t n, AncArgs a, const f
   }
 }
 
+// Units that begin an output row (their number is the number of rows hit).
+__global__ void k_count_rows(const uint32_t *row, uint64_t n, uint32_t *count) {
+  const uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t b = __ballot_sync(~0u, j < n && (j == 0 || row[j] != row[j - 1]));
+  if ((threadIdx.x & 31) == 0 && b != 0u) atomicAdd(count, (uint32_t)__popc(b));
+}
+
 // cut[s] = 1 + the row that the boundary before segment s cuts, or 0.
 __global__ void k_cut_rows(const uint32_t *row, uint32_t seg, uint32_t nsegs, uint32_t *cut) {
   const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -250,6 +257,7 @@ void pull_prepare(PullWalk &p, const DevCsf &c, int d, bool leaf, int R, int ldr
   p.leaf = leaf;
   p.n = c.nfibs[d];
   p.nsegs = 0;
+  p.every_row = false;
   if (p.n == 0) return;
   sort_by_row(c.fids[d].get(), p.n, c.dims[c.dim_perm[d]], p.perm, p.row, s);
   AncArgs a = {};
@@ -280,11 +288,17 @@ void pull_prepare(PullWalk &p, const DevCsf &c, int d, bool leaf, int R, int ldr
   p.nsegs = (uint32_t)((p.n + p.seg - 1) / p.seg);
   p.span.alloc((size_t)p.nsegs * 2 * ldr, s);
   ADATM_CUDA(cudaMemsetAsync(p.span.get(), 0, p.span.bytes(), s));  // padding columns stay zero
-  DevBuf<uint32_t> cut(p.nsegs, s);
+  DevBuf<uint32_t> cut(p.nsegs, s), hit(1, s);
+  ADATM_CUDA(cudaMemsetAsync(hit.get(), 0, sizeof(uint32_t), s));
+  k_count_rows<<<blocks_of(p.n), 256, 0, s>>>(p.row.get(), p.n, hit.get());
+  ADATM_LAUNCH();
+  uint32_t rows_hit = 0;
+  ADATM_CUDA(cudaMemcpyAsync(&rows_hit, hit.get(), sizeof(rows_hit), cudaMemcpyDeviceToHost, s));
   k_cut_rows<<<blocks_of(p.nsegs), 256, 0, s>>>(p.row.get(), p.seg, p.nsegs, cut.get());
   ADATM_LAUNCH();
   const int level = 0;
-  span_prepare(p.sums, cut.get(), 1, &level, p.nsegs, ldr, s);
+  span_prepare(p.sums, cut.get(), 1, &level, p.nsegs, ldr, s);  // (waits for the count as well)
+  p.every_row = rows_hit == c.dims[c.dim_perm[d]];
   if (leaf) p.perm.reset();
 }
 

@@ -21,6 +21,7 @@ struct PullWalk {
   DevBuf<uint32_t> anc[kMaxModes];  // factor row of the ancestor at levels 0 .. d-1
   DevBuf<double> span;           // head and tail row of every segment (ldr each)
   SpanSums sums;                 // of the rows that segment boundaries cut
+  bool every_row = false;        // every output row has units
 };
 
 // Sort level d's units by output row and look their ancestors up (device work).
