@@ -19,6 +19,8 @@ struct AlsWork {
   DevBuf<double> scalars;                // [0] ttnormsq, [1] fit, [2] norm, [3] inner
   DevBuf<int> iter;                      // ALS iteration counter (device)
   DevBuf<double> fit_trace;              // per-iteration fits
+  DevBuf<uint32_t> arrived;              // blocks of the launch under way that are done
+  int inner_blocks = 0;                  // rows of part_inner that the last inner update filled
   DevBuf<double> frob_part;              // partial sums of ||X||^2
   int max_trace = 0;
   void init(int nmodes_, int R_, int nblocks_, int max_iters, cudaStream_t s);
@@ -41,13 +43,16 @@ void gram(const float *A, uint64_t rows, int R, int ldr, double *G, AlsWork &w, 
 void frob_sq(const double *vals, uint64_t n, AlsWork &w, cudaStream_t s);
 // V = Hadamard of all G[n], n != mode; write V^-1 (fp64).
 void gram_inverse(const GramSet &g, int mode, AlsWork &w, cudaStream_t s);
-// A = normalize(M * V^-1) (M: the FP64 MTTKRP rows); updates lambda (2-norm on the first iteration,
-// max-norm floored at 1 afterwards), G_mode and, when `inner` is set, the
-// partial inner products <A, M> of the fit. A is fp32; with a bf16 copy (Ab
+// A = normalize(M * V^-1) (M: the FP64 MTTKRP rows); updates lambda (2-norm on
+// the first iteration, max-norm floored at 1 afterwards), G_mode and, when
+// `inner` is set, the partial inner products <A, M> of the fit, and with
+// fit_grams the fit itself, as fit() does. A is fp32; with a bf16 copy (Ab
 // non-null) the rows are rounded to bf16 in both copies and G_mode is taken
 // from the rounded rows.
 void update_factor(const double *M, uint64_t rows, float *A, __nv_bfloat16 *Ab, double *G_mode,
-                   bool inner, AlsWork &w, cudaStream_t s);
+                   bool inner, const GramSet *fit_grams, AlsWork &w, cudaStream_t s);
+// Kernel launches of update_factor without a separate fit.
+int update_kernels(uint64_t rows, bool bf16, const AlsWork &w);
 // fit = 1 - sqrt(||X||^2 + ||Z||^2 - 2<X,Z>) / ||X||, stored in
 // w.scalars[1] and w.fit_trace[iter]; advances w.iter.
 void fit(const GramSet &g, AlsWork &w, cudaStream_t s);
