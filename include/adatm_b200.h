@@ -229,8 +229,9 @@ int adatm_plan_splatt(const adatm_tensor *t, int csf_alloc, adatm_plan *out);
 
 /* Engine: trees, memo rows and factors for one plan and rank.
  * factor_bf16 != 0 keeps a BF16 copy of every factor for the gathers
- * (accumulation stays FP32). chunk_leaf/chunk_rows: source units per chunk
- * (0 = chosen from the number of units). The engine copies what it needs from the tensor. */
+ * (accumulation stays FP32). chunk_leaf/chunk_rows: source units per chunk, which
+ * the walkers of a contraction warp divide (0 = chosen from the number of units).
+ * The engine copies what it needs from the tensor. */
 int adatm_engine_create(const adatm_tensor *t, uint64_t rank, const adatm_plan *plan,
                         int factor_bf16, uint32_t chunk_leaf, uint32_t chunk_rows,
                         adatm_engine **out);
