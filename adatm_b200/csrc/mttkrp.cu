@@ -963,19 +963,26 @@ void find_hot_rows(TreeWalk &w, cudaStream_t s) {
 // Source units per chunk where the caller names none. A scatter's chunk is a
 // warp's; a contraction's is a walker's, and every walker slot of a resident
 // grid (4 blocks of 8 warps per SM) should have work: one chunk per slot while
-// that is at most kMaxChunk units (all slots then run once, side by side),
-// else chunks small enough that the last ones leave few slots idle.
+// that is at most kOnce units (all slots then run once, side by side), else
+// chunks small enough that the last ones leave few slots idle and no smaller
+// than their own sums pay for (fewer walkers per warp, wider rows: larger).
+// Above kOnce it is an eighth of a slot's share, at most 80 units, or 128 where
+// rows are wider than 32 columns.
 //
-// Measured (us per MTTKRP sequence, chunks of 16 / 32 / 64 / 128): 1M units,
-// R = 16 (26 units per slot) 154 / 145 / 154 / 187; 1.9M units, R = 24 (90
-// per slot) 451 / 404 / 391 / 373; 3.5M units, R = 32 (185 per slot) 955 /
-// 874 / 869 / 939; 55K units, R = 16 140 / 165 / 215 / -.
+// Measured (us per MTTKRP sequence, chunks of 16 / 32 / 64 / 96 / 128): 1M
+// units, R = 16 (26 units per slot) 98 / 83 / 93 / 116 / 128; 3.5M units, R = 32
+// (185 per slot) 672 / 666 / 760 / 812 / 926; 13M units, R = 32 (700 per slot)
+// 935 / 809 / 790 / 812 / 839; 70M units, R = 32 7352 / 6552 / 6291 / 6273 / 6303;
+// 3.4M units, R = 100 (740 per slot) 854 / 707 / 676 / 671 / 690; 40M units, R =
+// 64 6198 / 4960 / 4612 / 4532 / 4487. One chunk per slot against the best of
+// these: 1.9M units, R = 24 (101 per slot) 205 / 220.
 uint32_t auto_chunk(const TreeWalk &w) {
   if (w.src == w.out) return w.src == w.nmodes - 1 ? 2 * kScatterChunk : kScatterChunk;
-  constexpr uint64_t kMaxChunk = 128, kMinChunk = 16;
+  constexpr uint64_t kOnce = 128, kMinChunk = 16;
+  const uint64_t most = w.R <= 32 ? 80 : 128;
   const uint64_t slots = 148ull * 32 * default_walkers(w.R);
   const uint64_t per_slot = (w.nunits + slots - 1) / slots;
-  const uint64_t c = per_slot <= kMaxChunk ? per_slot : std::min(kMaxChunk, per_slot / 4);
+  const uint64_t c = per_slot <= kOnce ? per_slot : std::min(most, per_slot / 8);
   return (uint32_t)std::max(kMinChunk, (c + 15) / 16 * 16);
 }
 
