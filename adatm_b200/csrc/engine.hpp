@@ -19,13 +19,13 @@ struct EngineOptions {
   uint32_t chunk_rows = 0;  // source units per chunk, memo-row sources (0 = by size)
   int max_iters = 1024;       // capacity of the device fit trace
   // contraction walks as a resident grid whose warps claim chunks (fastest
-  // for one tensor on the device); off, one chunk per warp, so the blocks of
+  // for one tensor on the device); off, a group of chunks per warp, so the blocks of
   // walks running side by side on other streams interleave
   bool resident_grid = true;
   // walkers per warp of the contractions (0 = default_walkers(R))
   int walkers = 0;
-  // unstored levels folded into the contraction source loop (0..2; -1 =
-  // as many as each tree's fan-out suggests)
+  // most unstored levels folded into the contraction source loop (0..2; -1 =
+  // as many as each tree's fan-out suggests, up to five)
   int fold = -1;
   // no float atomics (the default): every MTTKRP output and memo row is
   // summed in an order fixed by the tree, in FP64 across chunks, so sweeps
@@ -79,7 +79,7 @@ class Engine {
   float *factor(int m) { return A_[m]; }
 
   // MTTKRP of `mode` following the plan (tags 0/1/2) into out (dims x ldr
-  // FP64, zeroed here). Memo reuse (tag 1) expects the group's memo root to have
+  // FP64, every row written). Memo reuse (tag 1) expects the group's memo root to have
   // run on the current factors of the memoized levels.
   void mttkrp(int mode, double *out);
   // same, with the factor rows read in the given precision
