@@ -285,8 +285,17 @@ BatchSweep::~BatchSweep() {
   if (fork_) cudaEventDestroy(fork_);
 }
 
+// The engines' streams are not ordered with the batch's: what als_begin queues
+// on them (Grams, the iteration counter, the trace) comes after the sweeps
+// under way on the batch's stream, and before the next one there.
 void BatchSweep::begin() {
-  for (Engine *e : e_) e->als_begin();
+  ADATM_CUDA(cudaEventRecord(fork_, s_));
+  for (Engine *e : e_) ADATM_CUDA(cudaStreamWaitEvent(e->stream(), fork_, 0));
+  for (size_t i = 0; i < e_.size(); ++i) {
+    e_[i]->als_begin();
+    ADATM_CUDA(cudaEventRecord(join_[i], e_[i]->stream()));
+    ADATM_CUDA(cudaStreamWaitEvent(s_, join_[i], 0));
+  }
   if (exec_) return;
   ADATM_CUDA(cudaStreamBeginCapture(s_, cudaStreamCaptureModeThreadLocal));
   try {
