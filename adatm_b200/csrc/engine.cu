@@ -176,6 +176,7 @@ void Engine::drop_graph() {
   if (graph_) cudaGraphDestroy(graph_);
   graph_exec_ = nullptr;
   graph_ = nullptr;
+  ++generation_;
 }
 
 void Engine::set_chunks(uint32_t chunk_leaf, uint32_t chunk_rows) {
@@ -278,8 +279,7 @@ BatchSweep::BatchSweep(std::vector<Engine *> engines, cudaStream_t stream)
 }
 
 BatchSweep::~BatchSweep() {
-  if (exec_) cudaGraphExecDestroy(exec_);
-  if (graph_) cudaGraphDestroy(graph_);
+  drop_graph();
   for (auto ev : join_)
     if (ev) cudaEventDestroy(ev);
   if (fork_) cudaEventDestroy(fork_);
@@ -296,7 +296,27 @@ void BatchSweep::begin() {
     ADATM_CUDA(cudaEventRecord(join_[i], e_[i]->stream()));
     ADATM_CUDA(cudaStreamWaitEvent(s_, join_[i], 0));
   }
-  if (exec_) return;
+  if (stale()) capture();
+}
+
+void BatchSweep::drop_graph() {
+  if (exec_) cudaGraphExecDestroy(exec_);
+  if (graph_) cudaGraphDestroy(graph_);
+  exec_ = nullptr;
+  graph_ = nullptr;
+}
+
+bool BatchSweep::stale() const {
+  if (!exec_) return true;
+  for (size_t i = 0; i < e_.size(); ++i)
+    if (e_[i]->generation() != captured_[i]) return true;
+  return false;
+}
+
+void BatchSweep::capture() {
+  drop_graph();
+  captured_.clear();
+  for (Engine *e : e_) captured_.push_back(e->generation());
   ADATM_CUDA(cudaStreamBeginCapture(s_, cudaStreamCaptureModeThreadLocal));
   try {
     ADATM_CUDA(cudaEventRecord(fork_, s_));
@@ -317,12 +337,15 @@ void BatchSweep::begin() {
 }
 
 void BatchSweep::sweep() {
-  if (!exec_) throw BadInput("the batch has not begun");
+  if (captured_.empty()) throw BadInput("the batch has not begun");
+  if (stale()) capture();
   ADATM_CUDA(cudaGraphLaunch(exec_, s_));
 }
 
 float BatchSweep::time_sweeps(int count) {
   cudaEvent_t a, b;
+  if (captured_.empty()) throw BadInput("the batch has not begun");
+  if (stale()) capture();
   ADATM_CUDA(cudaEventCreate(&a));
   ADATM_CUDA(cudaEventCreate(&b));
   ADATM_CUDA(cudaStreamSynchronize(s_));

@@ -129,6 +129,9 @@ class Engine {
   void sweep();                          // one ALS iteration (graph replay if captured)
   void sweep_eager();                    // one ALS iteration, plain launches
   void capture_graph();
+  // Raised by every change after which a captured sweep must not run any more
+  // (its walks' buffers may be gone).
+  uint64_t generation() const { return generation_; }
   double fit_host();                     // last fit (synchronises)
   int iter_host();
   void fit_trace(double *host, int n);
@@ -191,6 +194,7 @@ class Engine {
   float *staging(size_t n);
   cudaGraph_t graph_ = nullptr;
   cudaGraphExec_t graph_exec_ = nullptr;
+  uint64_t generation_ = 0;
   void drop_graph();
   // Side stream for the Gram inverse of a mode, which overlaps that mode's
   // MTTKRP (it reads only the other modes' Grams); fork / join events.
@@ -218,7 +222,7 @@ class BatchSweep {
   BatchSweep(const BatchSweep &) = delete;
   BatchSweep &operator=(const BatchSweep &) = delete;
   void begin();                 // als_begin of every engine, then capture
-  void sweep();                 // one graph launch
+  void sweep();                 // one graph launch (captured again if an engine changed)
   float time_sweeps(int count); // CUDA events on the batch stream, ms total
   int kernels_per_sweep() const;
 
@@ -229,6 +233,10 @@ class BatchSweep {
   std::vector<cudaEvent_t> join_;
   cudaGraph_t graph_ = nullptr;
   cudaGraphExec_t exec_ = nullptr;
+  std::vector<uint64_t> captured_;  // the engines' generations in the graph
+  bool stale() const;
+  void capture();
+  void drop_graph();
 };
 
 }  // namespace adatm

@@ -45,3 +45,41 @@ def test_rounds_of_one_batch(gpu, R):
             assert e.fit() == w[k][0]["fit"], k
             assert same(e.get_factors(), w[k][1]), k
     b.free()
+
+
+def test_engines_changed_between_rounds(gpu):
+    """Chunk sizes, walkers, folds and the summation of an engine change after
+    its sweep was captured in a batch, which frees what the captured launches
+    point to; another batch takes the same engines."""
+    A = gpu
+    changes = [lambda e: e.autotune(((48, 32),), sweeps=1), lambda e: e.set_walkers(1), lambda e: e.set_fold(0),
+               lambda e: (e.set_deterministic(False), e.set_deterministic(True))]
+    lone, batched = pairs(A, 16), pairs(A, 16)
+    es = [e for _, e in batched]
+    b = A.BatchSweep(es)
+    for k in range(len(changes) + 1):
+        if k:
+            changes[k - 1](lone[k - 1][1])
+            changes[k - 1](es[k - 1])
+        for e in es:
+            e.init_factors(k)
+        b.begin()
+        b.time_sweeps(2)
+        for (_, f), e in zip(lone, es):
+            f.init_factors(k)
+            assert f.als(2)["fit"] == e.fit(), k
+            assert same(f.get_factors(), e.get_factors()), k
+    # a change between begin and the sweeps, by another batch of the engines
+    for e in es:
+        e.init_factors(9)
+    b.begin()
+    other = A.BatchSweep(es[:2])
+    b.time_sweeps(2)
+    for (_, f), e in zip(lone, es):
+        f.init_factors(9)
+        assert f.als(2)["fit"] == e.fit()
+        assert same(f.get_factors(), e.get_factors())
+    other.free()
+    b.free()
+    with pytest.raises(A.AdatmError):
+        A.BatchSweep(es[:1]).time_sweeps(1)
