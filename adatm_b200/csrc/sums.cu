@@ -179,6 +179,7 @@ __global__ void __launch_bounds__(128) k_span_sums(const __grid_constant__ SumAr
       if (n + 1u == children) *count = 0u;
     }
     n = __shfl_sync(mask, n, 0, Q);
+    __syncwarp(mask);  // the first lane's acquire holds for all (a shuffle orders nothing)
     return n + 1u == children;
   };
   if (ng > 1u) {
