@@ -69,6 +69,19 @@ constexpr int kBatch = 32;  // units per batch of a scatter or pull warp
 // node on (a unit's is the open node plus the closes of that level before
 // it), so their ids come with one coalesced load per level.
 //
+// Rounding: where several walkers share a warp, a batch's units are added to
+// one another first and the batch's sum then to the open node's (`held`). One
+// run over a chunk of c units is off by about u c / sqrt(3 N) of a row of N
+// units, runs of B by u sqrt((B^2 + c^2 / B) / 3 N). A unit's value is multiplied
+// into its first row before the others are: in a skewed tensor many units share
+// rows, and what a product of rows alone is off by would not average out. (Up
+// to three BF16 rows come first: their product is exact in FP32.) Errors of the
+// root walks against FP64, with one run and the value last / as here: the
+// 6th-order Zipf(1.3) tensor 3.4e-9, 4.6e-9, 8.7e-9 / 1.3e-9, 1.1e-9, 7.8e-10; the
+// 5th-order one, BF16 rows, 5.6e-9, 4.7e-9 / 1.8e-9, 2.2e-9. It costs these walks
+// 2.18, 2.04, 1.86 -> 2.23, 2.09, 1.90 ms and 2.26, 1.15 -> 2.33, 1.16 ms; with the
+// sum held in registers, 2.26, 2.11, 1.91 and 2.41, 1.19.
+//
 // A node of level top that closes leaves the unit loop: its sum is stored
 // (memo rows, outputs), or multiplied by its own factor row and added to the
 // open node of the level above, in shared memory, and so on up as far as the
@@ -89,6 +102,7 @@ constexpr int kBatch = 32;  // units per batch of a scatter or pull warp
 // per SM (2.46 / 2.48), two walkers of two columns per lane (3.26).
 // ---------------------------------------------------------------------------
 constexpr int kMaxFold = 5;
+constexpr uint32_t kNoneHeld = 1u << 31;
 
 template <int W>
 struct WalkShape {
@@ -99,15 +113,21 @@ struct WalkShape {
 
 // Shared memory of one warp: the batch's staged units (a uint4 per unit: its
 // row, its parent's row, its value twice, as the packed products take it;
-// the rows of the ancestors further up in X words; its close depth), one
-// spare slot per walker, so that walkers read different banks; the open nodes
-// (a word per lane) and open sums (VW columns per lane) of levels d .. top-1.
+// the rows of the ancestors further up in X words), one spare slot per walker,
+// so that walkers read different banks; the units' close depths (a byte each,
+// in the spare slot where they fit); the open nodes (a word per lane) and open
+// sums (VW columns per lane) of levels d .. top-1; level top's sum of the
+// batches before (several walkers).
 __host__ __device__ constexpr int stage_words(int F) { return F <= 1 ? 0 : (F == 2 ? 1 : (F == 3 ? 2 : 4)); }
+template <int W>
+__host__ __device__ constexpr size_t depth_bytes() {
+  return WalkShape<W>::B > (int)sizeof(uint4) ? (size_t)W * WalkShape<W>::B : 0;
+}
 template <int W, int VW, int F>
 __host__ __device__ constexpr size_t contract_warp_smem(int d, int top) {
   return (size_t)W * (WalkShape<W>::B + 1) * (sizeof(uint4) + stage_words(F) * sizeof(uint32_t)) / 16 * 16 + 16 +
-         (size_t)W * WalkShape<W>::B +
-         (size_t)(top > d ? top - d : 0) * 32 * (sizeof(uint32_t) + VW * sizeof(float));
+         depth_bytes<W>() + (size_t)(top > d ? top - d : 0) * 32 * (sizeof(uint32_t) + VW * sizeof(float)) +
+         (W > 1 ? 32 * VW * sizeof(float) : 0);
 }
 
 // What the unit loop reads: factor rows of the source and folded levels lie
@@ -141,11 +161,14 @@ __global__ void __launch_bounds__(256, 4)
   uint4 *const stage = reinterpret_cast<uint4 *>(wbase) + wk * (B + 1);
   uint32_t *const stage2 =
       reinterpret_cast<uint32_t *>(reinterpret_cast<uint4 *>(wbase) + W * (B + 1)) + wk * (B + 1) * X;
-  uint8_t *const scd = wbase + kStageBytes + wk * B;
+  uint8_t *const scd =
+      depth_bytes<W>() != 0 ? wbase + kStageBytes + wk * B : reinterpret_cast<uint8_t *>(stage + B);
   // open node and open sum of level l in {d .. top-1}: nodes[l * 32], carry[l * 32]
-  uint32_t *const nodes = reinterpret_cast<uint32_t *>(wbase + kStageBytes + W * B) + lane - d * 32;
+  uint32_t *const nodes = reinterpret_cast<uint32_t *>(wbase + kStageBytes + depth_bytes<W>()) + lane - d * 32;
   Row<VW> *const carry =
       reinterpret_cast<Row<VW> *>(nodes + (top > d ? top : d) * 32 - lane) + lane - d * 32;
+  // sum of the open level-top node in the batches before this one
+  Row<VW> *const held = carry + (size_t)(top > d ? top : d) * 32;
   const int col = li * VW;
   const bool act = col < a.R;
   constexpr int esz = FT == FactorType::F32 ? 4 : 2;
@@ -162,6 +185,8 @@ __global__ void __launch_bounds__(256, 4)
 
   // units whose rows are in flight together: as many as the registers hold
   constexpr int SB = VW <= 2 ? 4 : (F <= 3 ? 2 : 1);
+  // folded rows multiplied into the source row before the value is
+  constexpr int E = FT == FactorType::BF16 ? (F < 2 ? F : 2) : 0;
   // the first group of W chunks by the warp's place in the grid, the next
   // ones from a counter (a resident grid), claimed while the current one runs
   uint32_t group = blockIdx.x * kWarps + warp;
@@ -172,7 +197,7 @@ __global__ void __launch_bounds__(256, 4)
     const uint32_t chunk_id = group * W + wk;
     const bool live = chunk_id < a.nchunks;
     const uint32_t *sc = a.sched + (size_t)(live ? chunk_id : 0u) * (S + 1);
-    uint32_t part = sc[S];
+    uint32_t part = sc[S] | kNoneHeld;  // levels whose open node began before the chunk
     uint32_t nt = sc[top];
     uint32_t nf[F >= 1 ? F : 1];  // open nodes of the folded levels
 #pragma unroll
@@ -197,6 +222,10 @@ __global__ void __launch_bounds__(256, 4)
     // A unit closes level top and `more` levels above it.
     auto close = [&](uint32_t more) {
       Row<VW> x = acc;
+      if (W > 1 && !(part & kNoneHeld)) {
+        x = row_add(*held, x);
+        part |= kNoneHeld;
+      }
       acc = row_zero<VW>();
       const uint32_t id = idt;
       if (hot.top_keep) keep(top, hot.top_store, nt, id, x);
@@ -224,7 +253,6 @@ __global__ void __launch_bounds__(256, 4)
       }
       carry[l * 32] = c;
     };
-    uint32_t lastcd = 0u;
     const uint32_t u0 = live ? chunk_id * a.chunk : 0u;  // (units are numbered in 32 bits)
     const uint32_t left0 = live ? min(a.chunk, (uint32_t)a.nunits - u0) : 0u;
     for (uint32_t b0 = 0; b0 < a.chunk; b0 += B) {
@@ -310,9 +338,6 @@ __global__ void __launch_bounds__(256, 4)
           }
 #pragma unroll
           for (int q = 0; q < SB; ++q) {
-            Row<VW> x = raw_row<VW, FT>(g[q]);
-#pragma unroll
-            for (int f = 0; f < F; ++f) x = row_mul(x, raw_row<VW, FT>(t[q][f]));
             Row<VW> y;
             if constexpr (!LEAF) {
               y = raw_row<VW, FactorType::F32>(m[q]);
@@ -324,7 +349,16 @@ __global__ void __launch_bounds__(256, 4)
 #pragma unroll
               for (int i = 0; i < VW / 2; ++i) y.w[i] = v[q];
             }
-            if (FULL || k + q < cnt) row_fma(acc, x, y);
+            Row<VW> x = raw_row<VW, FT>(g[q]);
+#pragma unroll
+            for (int f = 0; f < E; ++f) x = row_mul(x, raw_row<VW, FT>(t[q][f]));
+            if constexpr (F > E) {
+              y = row_mul(y, x);
+#pragma unroll
+              for (int f = E; f + 1 < F; ++f) y = row_mul(y, raw_row<VW, FT>(t[q][f]));
+              x = raw_row<VW, FT>(t[q][F - 1]);
+            }
+            if (FULL || k + q < cnt) row_fma(acc, y, x);
             if ((any >> (k + q)) & 1u) {
               if ((mt >> (k + q)) & 1u) close((uint32_t)scd[k + q] - (uint32_t)(F + 1));
               __syncwarp();
@@ -334,13 +368,20 @@ __global__ void __launch_bounds__(256, 4)
       };
       if (__all_sync(~0u, cnt == B)) run(std::true_type{});
       else run(std::false_type{});
-      if (cnt > 0) lastcd = scd[cnt - 1];
+      if (W > 1 && b0 + B < a.chunk) {
+        if (!(part & kNoneHeld)) acc = row_add(*held, acc);
+        *held = acc;
+        part &= ~kNoneHeld;
+        acc = row_zero<VW>();
+      }
       __syncwarp();
     }
     // chunk end: the nodes that the last unit did not close go on in the next
     // chunk; their partial sums go to the tail rows, or into their parents'
     if (live) {
-      Row<VW> x = acc;  // what the level holds, with what the level below adds
+      const uint32_t lastcd = __ldg(a.src_cd + (u0 + left0 - 1u));
+      // what the level holds, with what the level below adds
+      Row<VW> x = W > 1 && !(part & kNoneHeld) ? row_add(*held, acc) : acc;
       for (int l = top; l >= d; --l) {
         if (l < top) x = row_add(x, carry[l * 32]);
         if (l < S - (int)lastcd) {

@@ -151,8 +151,18 @@ __global__ void __launch_bounds__(256, 4) k_pull(const __grid_constant__ PullArg
           Row<4> x;
           if constexpr (LEAF) x.w[0] = x.w[1] = pack2(v[q], v[q]);
           else x = raw_row<4, FactorType::F32>(m[q]);
+          // the value or source row times the nearest ancestor's row first: units
+          // that share ancestors then do not share the rounding of a product of
+          // theirs; up to three BF16 rows come first, their product is exact
+          if constexpr (FT == FactorType::BF16 && DD >= 2) {
+            Row<4> e = raw_row<4, FT>(t[q][0]);
 #pragma unroll
-          for (int f = 0; f < DD; ++f) x = row_mul(x, raw_row<4, FT>(t[q][f]));
+            for (int f = 1; f < DD; ++f) e = row_mul(e, raw_row<4, FT>(t[q][f]));
+            x = row_mul(x, e);
+          } else {
+#pragma unroll
+            for (int f = 0; f < DD; ++f) x = row_mul(x, raw_row<4, FT>(t[q][f]));
+          }
           if constexpr (D > 3)
 #pragma unroll
             for (int f = 3; f < 7; ++f)
