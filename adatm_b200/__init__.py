@@ -839,6 +839,12 @@ class BatchSweep:
             pass
 
 
+def trim_memory():
+    """Give the device memory kept for reuse (512 MiB at most, while a tensor,
+    tree or engine is open) back to the device."""
+    _check(lib().adatm_trim_memory(), "adatm_trim_memory")
+
+
 def gram_device(A_ptr, rows, R, ldr, G_ptr):
     """G = A^T A (FP64) for a device row matrix; pointers are device addresses
     (e.g. torch tensor .data_ptr())."""

@@ -117,6 +117,7 @@ _SIGS = [
     ("adatm_free_groups", None, [C.POINTER(GroupProperties), u64]),
     ("adatm_last_error", C.c_char_p, []),
     ("adatm_set_device", C.c_int, [C.c_int]),
+    ("adatm_trim_memory", C.c_int, []),
     ("adatm_tensor_from_coo", C.c_int, [C.c_int, u64, P_u64, C.POINTER(P_u64), P_f64, C.c_int,
                                         C.POINTER(C.c_void_p)]),
     ("adatm_tensor_generate", C.c_int, [C.c_int, P_u64, u64, P_f64, C.c_int, C.c_double,

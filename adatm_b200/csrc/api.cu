@@ -429,6 +429,10 @@ int adatm_set_device(int device) {
   return guarded([&] { ADATM_CUDA(cudaSetDevice(device)); });
 }
 
+int adatm_trim_memory(void) {
+  return guarded([] { dev_trim(); });
+}
+
 // ---------------------------------------------------------------------------
 // options
 // ---------------------------------------------------------------------------

@@ -116,6 +116,12 @@ void dev_free(void *ptr) {
   while (p.kept_bytes > kPoolKept) give_back(p, p.kept.begin());
 }
 
+void dev_trim() {
+  Pool &p = pool();
+  std::lock_guard<std::mutex> lk(p.mu);
+  while (!p.kept.empty()) give_back(p, p.kept.begin());
+}
+
 void stream_opened(cudaStream_t s) {
   std::lock_guard<std::mutex> lk(pool().mu);
   pool().streams.insert(s);

@@ -10,8 +10,9 @@
 // its size on the same stream, which the stream itself orders; when the stream
 // is closed, it is waited for and its buffers are free for any stream. The
 // pool keeps at most kPoolKept bytes, gives the oldest back beyond that, gives
-// everything back when an allocation fails or when the last stream closes,
-// and takes no block above kPoolBlock. Buffers without a stream, or of a
+// everything back when one of its own allocations fails, when the last stream
+// closes or when it is told to (dev_trim: the memory is missing to somebody
+// else), and takes no block above kPoolBlock. Buffers without a stream, or of a
 // stream that is not the library's, go straight to cudaMalloc and cudaFree.
 #pragma once
 
@@ -28,6 +29,7 @@ constexpr size_t kPoolKept = (size_t)512 << 20;
 
 void *dev_alloc(size_t bytes, cudaStream_t stream);
 void dev_free(void *p);
+void dev_trim();
 
 // A stream that buffers may be taken for, from its creation to just before its
 // destruction.

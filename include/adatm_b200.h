@@ -200,6 +200,13 @@ const char *adatm_last_error(void);
  * CUDA runtime, so a framework's device selection does not reach it). */
 int adatm_set_device(int device);
 
+/* Give the device memory that the library keeps for reuse back to the device.
+ * While a tensor, tree or engine handle is open, buffers of freed engines and
+ * of finished set-up work (up to 64 MiB each, 512 MiB in all) are kept; they go
+ * back by themselves when an allocation of the library fails and when the last
+ * handle is freed. For a host whose own allocator runs out in between. */
+int adatm_trim_memory(void);
+
 /* COO tensor into HBM. With clean != 0, duplicates are summed in input order
  * and empty slices of every mode are compacted (dims shrink accordingly). */
 int adatm_tensor_from_coo(int nmodes, uint64_t nnz, const uint64_t *dims,
