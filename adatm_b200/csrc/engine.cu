@@ -433,7 +433,10 @@ void Engine::check_use(int mode, int tree, int tag) const {
   }
 }
 
-std::unique_ptr<TreeWalk> Engine::make_walk(int mode, int g, int tag) {
+// of_plan: one of the plan's walks, for which the shared scratch may still grow.
+// Captured sweeps point to it, so it must not grow for a walk that is made
+// later: such a walk takes a scratch of its own where the shared one is too small.
+std::unique_ptr<TreeWalk> Engine::make_walk(int mode, int g, int tag, bool of_plan) {
   const int N = coo_->nmodes;
   const DevCsf &c = *csf_[g];
   const Group &gp = plan_.tree(g);
@@ -462,14 +465,17 @@ std::unique_ptr<TreeWalk> Engine::make_walk(int mode, int g, int tag) {
     }
   }
   walk_prepare(*w, stream_);
+  w->scratch = of_plan || scratch_->holds(*w) ? scratch_ : std::make_shared<WalkScratch>();
+  w->scratch->reserve(*w, stream_);
   return w;
 }
 
 void Engine::build_walks() {
   custom_.clear();
+  scratch_ = std::make_shared<WalkScratch>();
   for (int m = 0; m < coo_->nmodes; ++m) {
     const int g = (int)plan_.use_csfs[m];
-    walk_[m] = make_walk(m, g, (int)plan_.use_tags[m]);
+    walk_[m] = make_walk(m, g, (int)plan_.use_tags[m], true);
     direct_[m].reset();  // built on first use (mttkrp_direct)
   }
 }
@@ -506,7 +512,7 @@ void Engine::mttkrp_with(int mode, int tree, int tag, double *out) {
     w = walk_[mode].get();
   } else {
     auto &slot = custom_[std::make_tuple(mode, tree, tag)];
-    if (!slot) slot = make_walk(mode, tree, tag);
+    if (!slot) slot = make_walk(mode, tree, tag, false);
     w = slot.get();
   }
   clear_output(*w, mode, out);
@@ -548,7 +554,7 @@ FactorType Engine::sweep_type(int mode) const {
 }
 
 void Engine::mttkrp_direct(int mode, double *out) {
-  if (!direct_[mode]) direct_[mode] = make_walk(mode, (int)plan_.use_csfs[mode], 2);
+  if (!direct_[mode]) direct_[mode] = make_walk(mode, (int)plan_.use_csfs[mode], 2, false);
   clear_output(*direct_[mode], mode, out);
   walk_launch(*direct_[mode], level_factors((int)plan_.use_csfs[mode], opt_.factor_type),
               opt_.factor_type, out, stream_);

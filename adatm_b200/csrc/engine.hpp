@@ -166,7 +166,7 @@ class Engine {
 
  private:
   void build_walks();
-  std::unique_ptr<TreeWalk> make_walk(int mode, int tree, int tag);
+  std::unique_ptr<TreeWalk> make_walk(int mode, int tree, int tag, bool of_plan);
   LevelFactors level_factors(int g, FactorType ft) const;
   void clear_output(const TreeWalk &w, int mode, double *out);
 
@@ -178,6 +178,7 @@ class Engine {
   cudaStream_t stream_;
   std::vector<std::shared_ptr<DevCsf>> csf_;
   DevBuf<float> memo_[kMaxModes][kMaxModes];
+  std::shared_ptr<WalkScratch> scratch_;  // of the plan's walks, and of others that it holds
   std::unique_ptr<TreeWalk> walk_[kMaxModes];
   std::unique_ptr<TreeWalk> direct_[kMaxModes];
   std::map<std::tuple<int, int, int>, std::unique_ptr<TreeWalk>> custom_;  // by (mode, tree, tag)

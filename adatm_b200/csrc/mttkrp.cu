@@ -659,6 +659,11 @@ __global__ void k_cut_nodes(WalkArgs a, uint32_t *cut) {
       cut[(size_t)a.span_lev[l] * a.nchunks + c] = (sc[a.S] >> l) & 1u ? sc[l] + 1u : 0u;
 }
 
+// Memo rows of level l, or the scratch rows of a contraction's level-d sums.
+float *store_of(const TreeWalk &w, int l) {
+  return l == w.out && w.level_store() && w.scratch ? w.scratch->level_rows.get() : w.store[l];
+}
+
 WalkArgs make_args(const TreeWalk &w, const LevelFactors *f, double *out) {
   WalkArgs a;
   const DevCsf &c = *w.csf;
@@ -676,7 +681,7 @@ WalkArgs make_args(const TreeWalk &w, const LevelFactors *f, double *out) {
     a.fptr[l] = c.fptr[l].get();
     a.fids[l] = c.fids[l].get();
     a.U[l] = f ? f->U[l] : nullptr;
-    a.store[l] = w.store[l];
+    a.store[l] = store_of(w, l);
   }
   a.vals = c.vals32.get();
   a.src_rows = w.src_rows;
@@ -688,7 +693,7 @@ WalkArgs make_args(const TreeWalk &w, const LevelFactors *f, double *out) {
   a.nhot = w.nhot;
   a.hot_slot = w.hot_slot.get();
   a.hot_rows = w.hot_rows.get();
-  a.span = w.span_nlev > 0 ? w.span.get() : nullptr;
+  a.span = w.span_nlev > 0 && w.scratch ? w.scratch->span.get() : nullptr;
   a.span_nlev = w.span_nlev;
   for (int l = 0; l < kMaxModes; ++l) a.span_lev[l] = w.span_lev[l];
   return a;
@@ -921,11 +926,8 @@ void prepare_spans(TreeWalk &w, cudaStream_t s) {
   const DevCsf &c = *w.csf;
   const int S = w.src, d = w.out;
   if (d > 0) {
-    // the level-d sums are stored, then pulled (or, with atomics, scattered)
-    // into the output rows
-    w.level_rows.alloc((size_t)std::max<uint64_t>(c.nfibs[d], 1) * w.ldr, s);
-    ADATM_CUDA(cudaMemsetAsync(w.level_rows.get(), 0, w.level_rows.bytes(), s));
-    w.store[d] = w.level_rows.get();
+    // the level-d sums are stored (level_store), then pulled (or, with atomics,
+    // scattered) into the output rows
     if (!w.deterministic) {
       w.scatter = std::make_unique<TreeWalk>();
       TreeWalk &t = *w.scatter;
@@ -933,7 +935,6 @@ void prepare_spans(TreeWalk &w, cudaStream_t s) {
       t.R = w.R;
       t.ldr = w.ldr;
       t.src = t.out = d;
-      t.src_rows = w.level_rows.get();
       t.chunk = kScatterChunk;
       walk_prepare(t, s);
     }
@@ -941,10 +942,8 @@ void prepare_spans(TreeWalk &w, cudaStream_t s) {
   w.span_nlev = 0;
   for (int l = 0; l < kMaxModes; ++l) w.span_lev[l] = -1;
   for (int l = 0; l < S; ++l)
-    if (w.store[l] != nullptr || (l == 0 && d == 0)) w.span_lev[l] = w.span_nlev++;
+    if (w.stores(l) || (l == 0 && d == 0)) w.span_lev[l] = w.span_nlev++;
   if (w.nchunks == 0 || w.span_nlev == 0) return;
-  w.span.alloc((size_t)w.nchunks * w.span_nlev * 2 * w.ldr, s);
-  ADATM_CUDA(cudaMemsetAsync(w.span.get(), 0, w.span.bytes(), s));  // padding columns stay zero
   DevBuf<uint32_t> cut((size_t)w.span_nlev * w.nchunks, s);
   k_cut_nodes<<<(w.nchunks + 255) / 256, 256, 0, s>>>(make_args(w, nullptr, nullptr), cut.get());
   ADATM_LAUNCH();
@@ -956,10 +955,10 @@ void prepare_spans(TreeWalk &w, cudaStream_t s) {
 
 void launch_sums(const TreeWalk &w, double *out, cudaStream_t s) {
   SpanTarget t;
-  for (int l = 0; l < kMaxModes; ++l) t.store[l] = w.store[l];
+  for (int l = 0; l < kMaxModes; ++l) t.store[l] = store_of(w, l);
   t.out = w.out == 0 ? out : nullptr;
   t.out_ids = w.csf->fids[0].get();
-  span_launch<float>(w.sums, w.span.get(), w.span_nlev, w.R, w.ldr, t, s);
+  span_launch<float>(w.sums, w.scratch->span.get(), w.span_nlev, w.R, w.ldr, t, s);
 }
 
 }  // namespace
@@ -1008,22 +1007,31 @@ void find_hot_rows(TreeWalk &w, cudaStream_t s) {
 // chunks small enough that the last ones leave few slots idle and no smaller
 // than their own sums pay for (fewer walkers per warp, wider rows: larger).
 // Above kOnce it is an eighth of a slot's share, at most 80 units, or 128 where
-// rows are wider than 32 columns.
+// rows are wider than 32 columns. Nonzeros that give every slot more than 64
+// such chunks take larger ones, up to 256 units: the head and tail rows of a
+// chunk (two rows for every spanned level) then take no more memory per
+// nonzero than chunks of 256 do, where a tensor comes near the device's size.
 //
 // Measured (us per MTTKRP sequence, chunks of 16 / 32 / 64 / 96 / 128): 1M
 // units, R = 16 (26 units per slot) 98 / 83 / 93 / 116 / 128; 3.5M units, R = 32
 // (185 per slot) 672 / 666 / 760 / 812 / 926; 13M units, R = 32 (700 per slot)
 // 935 / 809 / 790 / 812 / 839; 70M units, R = 32 7352 / 6552 / 6291 / 6273 / 6303;
 // 3.4M units, R = 100 (740 per slot) 854 / 707 / 676 / 671 / 690; 40M units, R =
-// 64 6198 / 4960 / 4612 / 4532 / 4487. One chunk per slot against the best of
-// these: 1.9M units, R = 24 (101 per slot) 205 / 220.
+// 64 6198 / 4960 / 4612 / 4532 / 4487. Around kOnce, one root walk of R = 32,
+// chunks of 16 / 32 / 64 / 128 / one per slot: 97 per slot 66 / 70 / 86 / 81 / 78; 120
+// 76 / 79 / 87 / 84 / 84; 130 79 / 82 / 95 / 109 / -; 208 115 / 110 / 122 / 143 / -; R = 64,
+// 122 per slot 71 / 67 / 68 / 65 / 65; 132 74 / 70 / 73 / 86 / -. The 78M-nonzero
+// tensor (4112 per slot) with 80 / 112 / 256: 6405, 6425, 6670; at 256 units a slot
+// has 16 chunks there, and 64 where the rule names 256.
 uint32_t auto_chunk(const TreeWalk &w) {
   if (w.src == w.out) return w.src == w.nmodes - 1 ? 2 * kScatterChunk : kScatterChunk;
   constexpr uint64_t kOnce = 128, kMinChunk = 16;
-  const uint64_t most = w.R <= 32 ? 80 : 128;
+  const uint64_t most = w.R <= 32 ? 80 : 128, large = w.src == w.nmodes - 1 ? 256 : most;
   const uint64_t slots = 148ull * 32 * default_walkers(w.R);
   const uint64_t per_slot = (w.nunits + slots - 1) / slots;
-  const uint64_t c = per_slot <= kOnce ? per_slot : std::min(most, per_slot / 8);
+  const uint64_t c = per_slot <= kOnce
+                         ? per_slot
+                         : std::max(std::min(most, per_slot / 8), std::min(large, per_slot / 64));
   return (uint32_t)std::max(kMinChunk, (c + 15) / 16 * 16);
 }
 
@@ -1064,14 +1072,35 @@ void walk_prepare(TreeWalk &w, cudaStream_t s) {
   if (!w.deterministic && w.src == w.out && w.nunits >= kHotMin) find_hot_rows(w, s);
 }
 
-void walk_launch(const TreeWalk &w, const LevelFactors &f, FactorType ft, double *out,
-                 cudaStream_t s) {
+bool WalkScratch::holds(const TreeWalk &w) const {
+  return span.n >= w.span_words() && level_rows.n >= w.level_words() && pull_span.n >= w.pull_words();
+}
+
+void WalkScratch::reserve(const TreeWalk &w, cudaStream_t s) {
+  auto grow = [&](auto &buf, size_t n) {
+    if (buf.n >= n) return;
+    std::decay_t<decltype(buf)> b(n, s);  // (the walks keep what they have if this throws)
+    ADATM_CUDA(cudaMemsetAsync(b.get(), 0, b.bytes(), s));
+    buf = std::move(b);
+  };
+  grow(span, w.span_words());
+  grow(level_rows, w.level_words());
+  grow(pull_span, w.pull_words());
+}
+
+namespace {
+
+// src_rows: the walk's source rows where they are not its own (scatter of a
+// contraction's sums).
+void launch(const TreeWalk &w, const LevelFactors &f, FactorType ft, const float *src_rows, double *out,
+            cudaStream_t s) {
   if (w.nchunks == 0) return;
   if (w.deterministic && w.src == w.out) {
-    pull_launch(*w.pull, f.U, ft, w.src_rows, out, s);
+    pull_launch(*w.pull, f.U, ft, src_rows, w.scratch->pull_span.get(), out, s);
     return;
   }
-  const WalkArgs a = make_args(w, &f, w.src > w.out && w.out > 0 ? nullptr : out);
+  WalkArgs a = make_args(w, &f, w.src > w.out && w.out > 0 ? nullptr : out);
+  a.src_rows = src_rows;
   const bool leaf = w.src == w.nmodes - 1;
   if (w.src > w.out) {
     const int wk = w.walkers > 0 ? w.walkers : default_walkers(w.R);
@@ -1083,8 +1112,9 @@ void walk_launch(const TreeWalk &w, const LevelFactors &f, FactorType ft, double
       else launch_contract<FactorType::BF16, false>(wk, w.fold, a, w.resident, s);
     }
     launch_sums(w, out, s);
-    if (w.scatter) walk_launch(*w.scatter, f, ft, out, s);
-    else if (w.pull) pull_launch(*w.pull, f.U, ft, w.level_rows.get(), out, s);
+    if (w.scatter) launch(*w.scatter, f, ft, w.scratch->level_rows.get(), out, s);
+    else if (w.pull)
+      pull_launch(*w.pull, f.U, ft, w.scratch->level_rows.get(), w.scratch->pull_span.get(), out, s);
   } else {
     const unsigned blocks = (unsigned)((w.nchunks + kWarps - 1) / kWarps);
     const int lanes = lanes_for_rank(w.R);
@@ -1096,6 +1126,12 @@ void walk_launch(const TreeWalk &w, const LevelFactors &f, FactorType ft, double
       else launch_scatter<FactorType::BF16, false>(lanes, a, blocks, s);
     }
   }
+}
+
+}  // namespace
+
+void walk_launch(const TreeWalk &w, const LevelFactors &f, FactorType ft, double *out, cudaStream_t s) {
+  launch(w, f, ft, w.src_rows, out, s);
 }
 
 bool walk_fills_output(const TreeWalk &w) {
@@ -1136,7 +1172,7 @@ double walk_compulsory_bytes(const TreeWalk &w, FactorType ft, const uint64_t *d
   for (int l = 0; l < N; ++l)
     if (l <= w.src && l != w.out) b += bf * R * (double)dims_of_level[l];  // factors
   for (int l = 0; l < kMaxModes; ++l)
-    if (w.store[l]) b += 4.0 * R * (double)c.nfibs[l];     // memo rows written
+    if (w.stores(l)) b += 4.0 * R * (double)c.nfibs[l];    // memo rows written
   b += 8.0 * R * (double)out_rows;                         // output (FP64 rows)
   return b;
 }

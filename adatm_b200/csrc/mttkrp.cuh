@@ -36,6 +36,19 @@ struct LevelFactors {
   const void *U[kMaxModes] = {nullptr};
 };
 
+// Rows that a walk writes and reads within one launch sequence: head and tail
+// rows of a contraction's chunks, the level-d sums of one below the root, head
+// and tail rows of a pull's segments. Walks that run one after another on one
+// stream share them. The padding columns, which no walk has to write, are zero.
+struct WalkScratch {
+  DevBuf<float> span;        // nchunks x span_nlev x 2 x ldr
+  DevBuf<float> level_rows;  // nodes of level d x ldr
+  DevBuf<double> pull_span;  // nsegs x 2 x ldr
+  bool holds(const struct TreeWalk &w) const;
+  // Room for w's rows as well (what was there is not kept).
+  void reserve(const struct TreeWalk &w, cudaStream_t s);
+};
+
 struct TreeWalk {
   int nmodes = 0;
   int src = 0;                 // source level S
@@ -71,16 +84,17 @@ struct TreeWalk {
   bool deterministic = false;
   int span_nlev = 0;
   int span_lev[kMaxModes] = {-1, -1, -1, -1, -1, -1, -1, -1};
-  DevBuf<float> span;                // nchunks x span_nlev x 2 x ldr
   SpanSums sums;
-  DevBuf<float> level_rows;          // contraction below the root: level-d node sums
-  std::unique_ptr<TreeWalk> scatter; // and, with atomics, their scatter into the output rows
+  std::unique_ptr<TreeWalk> scatter; // contraction below the root, with atomics: the
+                                     // scatter of its level-d sums into the output rows
   std::unique_ptr<PullWalk> pull;    // scatter of level `out` as a pull (deterministic)
-  bool has_store() const {
-    for (int l = 0; l < kMaxModes; ++l)
-      if (store[l]) return true;
-    return false;
-  }
+  std::shared_ptr<WalkScratch> scratch;  // set before the first launch
+  // contraction below the root: its level-d sums are rows of the scratch
+  bool level_store() const { return src > out && out > 0; }
+  bool stores(int l) const { return store[l] != nullptr || (l == out && level_store()); }
+  size_t span_words() const { return (size_t)nchunks * span_nlev * 2 * ldr; }
+  size_t level_words() const { return level_store() ? (size_t)csf->nfibs[out] * ldr : 0; }
+  size_t pull_words() const { return pull ? pull->span_words() : 0; }
 };
 
 // Kernel launches of one walk (for launch counts).

@@ -291,13 +291,14 @@ void pull_prepare(PullWalk &p, const DevCsf &c, int d, bool leaf, int R, int ldr
   k_ancestors<<<blocks_of(p.n), 256, 0, s>>>(p.perm.get(), p.n, a, c.vals32.get(), leaf ? p.vals.get() : nullptr);
   ADATM_LAUNCH();
   // segments: one per walker slot of a full device while that is at most 128
-  // units, else short enough that the last ones leave few slots idle
+  // units, else short enough that the last ones leave few slots idle. Leaf
+  // pulls, us with 16 / 32 / 64 / 128 / one per slot: R = 32, 97 units per slot 61 /
+  // 62 / 61 / 65 / 61; 120 75 / 72 / 67 / 68 / 68; 130 78 / 76 / 75 / 84 / -; 208 115 / 112 /
+  // 113 / 105 / -; 460 238 / 212 / 209 / 209 / -; R = 64, 132 per slot 76 / 70 / 73 / 84 / -
   const uint64_t slots = 148ull * 32 * walkers_of(R), per_slot = (p.n + slots - 1) / slots;
   const uint64_t u = per_slot <= 128 ? per_slot : std::min<uint64_t>(128, per_slot / 4);
   p.seg = (uint32_t)std::max<uint64_t>(16, (u + 15) / 16 * 16);
   p.nsegs = (uint32_t)((p.n + p.seg - 1) / p.seg);
-  p.span.alloc((size_t)p.nsegs * 2 * ldr, s);
-  ADATM_CUDA(cudaMemsetAsync(p.span.get(), 0, p.span.bytes(), s));  // padding columns stay zero
   DevBuf<uint32_t> cut(p.nsegs, s), hit(1, s);
   ADATM_CUDA(cudaMemsetAsync(hit.get(), 0, sizeof(uint32_t), s));
   k_count_rows<<<blocks_of(p.n), 256, 0, s>>>(p.row.get(), p.n, hit.get());
@@ -312,8 +313,8 @@ void pull_prepare(PullWalk &p, const DevCsf &c, int d, bool leaf, int R, int ldr
   if (leaf) p.perm.reset();
 }
 
-void pull_launch(const PullWalk &p, const void *const *U, FactorType ft, const float *src_rows, double *out,
-                 cudaStream_t s) {
+void pull_launch(const PullWalk &p, const void *const *U, FactorType ft, const float *src_rows, double *span,
+                 double *out, cudaStream_t s) {
   if (p.nsegs == 0) return;
   PullArgs a = {};
   a.d = p.d;
@@ -331,7 +332,7 @@ void pull_launch(const PullWalk &p, const void *const *U, FactorType ft, const f
   }
   a.src_rows = src_rows;
   a.out = out;
-  a.span = p.span.get();
+  a.span = span;
   if (ft == FactorType::F32) {
     if (p.leaf) launch_w<FactorType::F32, true>(a, s);
     else launch_w<FactorType::F32, false>(a, s);
@@ -341,7 +342,7 @@ void pull_launch(const PullWalk &p, const void *const *U, FactorType ft, const f
   }
   SpanTarget t;
   t.out = out;
-  span_launch<double>(p.sums, p.span.get(), 1, p.R, p.ldr, t, s);
+  span_launch<double>(p.sums, span, 1, p.R, p.ldr, t, s);
 }
 
 int pull_kernels(const PullWalk &p) { return p.nsegs ? 1 + span_kernels(p.sums) : 0; }

@@ -19,9 +19,9 @@ struct PullWalk {
   DevBuf<float> vals;            // value (leaf sources)
   DevBuf<uint32_t> row;          // output row
   DevBuf<uint32_t> anc[kMaxModes];  // factor row of the ancestor at levels 0 .. d-1
-  DevBuf<double> span;           // head and tail row of every segment (ldr each)
   SpanSums sums;                 // of the rows that segment boundaries cut
   bool every_row = false;        // every output row has units
+  size_t span_words() const { return (size_t)nsegs * 2 * ldr; }
 };
 
 // Sort level d's units by output row and look their ancestors up (device work).
@@ -29,8 +29,9 @@ void pull_prepare(PullWalk &p, const DevCsf &c, int d, bool leaf, int R, int ldr
 
 // out[row] = sum over the row's units of src(unit) times the factor rows of
 // its ancestors (U: factor rows per level); rows without units are left alone.
-void pull_launch(const PullWalk &p, const void *const *U, FactorType ft, const float *src_rows, double *out,
-                 cudaStream_t s);
+// span: head and tail row of every segment (span_words(), padding columns zero).
+void pull_launch(const PullWalk &p, const void *const *U, FactorType ft, const float *src_rows, double *span,
+                 double *out, cudaStream_t s);
 
 int pull_kernels(const PullWalk &p);
 

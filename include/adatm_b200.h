@@ -340,9 +340,10 @@ int adatm_engine_set_fold(adatm_engine *e, int fold);
  * output level is below the root, visit every output row's contributions in
  * a stable order by row. Output rows are FP64 sums. Sweeps then repeat bit
  * for bit from the same start, on one device and build. Costs extra device
- * memory (per-chunk rows, sorted unit lists, prefix rows). Off (on == 0),
+ * memory (sorted unit lists with the rows of their ancestors). Off (on == 0),
  * scatters add into the FP64 output rows with atomics (order-dependent in
- * the last bits). Drops a captured sweep. No reference counterpart: the
+ * the last bits). Either way an engine keeps per-chunk rows and, for walks
+ * below the root, the sums of the output level's nodes, once for all walks. Drops a captured sweep. No reference counterpart: the
  * reference's locked OpenMP scatters (mttkrp.c:13-14,121-125) sum in thread
  * order. */
 int adatm_engine_set_deterministic(adatm_engine *e, int on);
