@@ -202,6 +202,11 @@ void Engine::set_walkers(int walkers) {
                    std::to_string(R_));
   drop_graph();
   opt_.walkers = walkers;
+  if (opt_.chunk_leaf != 0 || opt_.chunk_rows != 0) {  // the walkers divide a named chunk
+    build_walks();
+    ADATM_CUDA(cudaStreamSynchronize(stream_));
+    return;
+  }
   for (int m = 0; m < coo_->nmodes; ++m) {
     walk_[m]->walkers = walkers;
     if (direct_[m]) direct_[m]->walkers = walkers;

@@ -1040,8 +1040,8 @@ uint32_t auto_chunk(const TreeWalk &w) {
 // walker, large chunks leave most slots of a small tensor's grid idle. us per
 // MTTKRP sequence, whole / divided, chunks of 256 and 1024: 20K nonzeros, R = 16
 // 166 / 57 and 492 / 101; 3.5M nonzeros, R = 32 1002 / 759 and 2881 / 998.
-uint32_t walker_chunk(uint32_t chunk, int R) {
-  const uint32_t W = (uint32_t)default_walkers(R);
+uint32_t walker_chunk(uint32_t chunk, int walkers) {
+  const uint32_t W = (uint32_t)walkers;
   return std::max(std::min(chunk, 16u), chunk / W + (chunk % W != 0));
 }
 
@@ -1053,7 +1053,7 @@ void walk_prepare(TreeWalk &w, cudaStream_t s) {
   if (w.chunk == 0)
     w.chunk = auto_chunk(w);
   else if (w.src > w.out)
-    w.chunk = walker_chunk(w.chunk, w.R);
+    w.chunk = walker_chunk(w.chunk, w.walkers > 0 ? w.walkers : default_walkers(w.R));
   w.chunk = std::min(w.chunk, 1u << 30);  // offsets in a chunk are 32-bit numbers
   w.nchunks = (uint32_t)((w.nunits + w.chunk - 1) / w.chunk);
   w.sched.alloc((size_t)std::max<uint32_t>(w.nchunks, 1) * (w.src + 1) + 1, s);  // + the chunk counter
