@@ -745,9 +745,10 @@ class Engine:
         _check(lib().adatm_engine_launch_counts(self._h, mode, C.byref(a), C.byref(b)), "launch_counts")
         return a.value, b.value
 
-    def autotune(self, options=((128, 64), (256, 128), (512, 256), (1024, 512)), sweeps=3):
+    def autotune(self, options=((0, 0), (128, 64), (256, 128), (512, 256), (1024, 512)), sweeps=3):
         """Keep the fastest (chunk_leaf, chunk_rows) of `options` by timing a
-        captured sweep of each; returns its index. Initialise the factors
+        captured sweep of each; returns its index. (0, 0) stands for the sizes
+        that an engine has without being told any. Initialise the factors
         afterwards."""
         leaf = (C.c_uint32 * len(options))(*[o[0] for o in options])
         rows = (C.c_uint32 * len(options))(*[o[1] for o in options])

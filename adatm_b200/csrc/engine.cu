@@ -180,7 +180,6 @@ void Engine::drop_graph() {
 }
 
 void Engine::set_chunks(uint32_t chunk_leaf, uint32_t chunk_rows) {
-  if (chunk_leaf == 0 || chunk_rows == 0) throw BadInput("chunk sizes must be positive");
   drop_graph();
   opt_.chunk_leaf = chunk_leaf;
   opt_.chunk_rows = chunk_rows;

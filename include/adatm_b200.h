@@ -305,7 +305,8 @@ int adatm_engine_hot_rows(adatm_engine *e, uint64_t mode, int *nhot);
 /* ------------------------------------------------------------------------ */
 
 /* Time a captured sweep with each (chunk_leaf[i], chunk_rows[i]) and keep the
- * fastest (*best = its index). Runs sweeps: initialise the factors after. */
+ * fastest (*best = its index). A size of 0 is chosen from the number of units,
+ * as in adatm_engine_create. Runs sweeps: initialise the factors after. */
 int adatm_engine_autotune(adatm_engine *e, const uint32_t *chunk_leaf, const uint32_t *chunk_rows,
                           int n, int sweeps, int *best);
 

@@ -32,3 +32,31 @@ def test_named_chunks_are_divided_among_the_walkers_set(gpu, walkers):
     a.free()
     b.free()
     t.free()
+
+
+def test_autotuning_can_keep_the_automatic_sizes(gpu):
+    """(0, 0) is among the options, and tuning to it alone gives back the engine
+    that was there before: every sum, bit for bit."""
+    A = gpu
+    t = A.Tensor.generate([400, 300, 200, 100], 80000, alpha=1.2, seed=7)
+    plan = A.plan_analytic(t, 16)[0]
+    mats = O.init_factors(t.info()[2], 16, 3)
+    e = A.Engine(t, 16, plan)
+    e.set_factors(mats)
+    want = [e.mttkrp(m) for m in range(4)]
+    e.autotune(((512, 512),), sweeps=1)
+    e.set_factors(mats)
+    assert not all(np.array_equal(e.mttkrp(m), w) for m, w in enumerate(want))
+    assert e.autotune(((0, 0),), sweeps=1) == 0
+    e.set_factors(mats)
+    assert all(np.array_equal(e.mttkrp(m), w) for m, w in enumerate(want))
+    assert e.autotune() in range(5)
+    e.free()
+    t.free()
+
+
+def test_default_options_name_the_automatic_sizes():
+    import inspect
+
+    import adatm_b200 as A
+    assert (0, 0) in inspect.signature(A.Engine.autotune).parameters["options"].default
