@@ -759,7 +759,7 @@ class Engine:
 
     def set_resident_grid(self, on):
         """Contraction walks as a resident grid claiming chunks (True, the
-        default) or one chunk per warp (False, as in a batch)."""
+        default) or one group of chunks per warp (False, as in a batch)."""
         _check(lib().adatm_engine_set_resident_grid(self._h, int(bool(on))),
                "adatm_engine_set_resident_grid")
 

@@ -1,7 +1,7 @@
 // als.cuh -- the dense part of one CP-ALS mode update on the GPU
 // (cpd_als_iterate_adaptive, adatm_cpd.c:320-335, and the fit,
 // adatm_cpd.c:59-200). FP64 is kept for the R x R Gram Hadamard product, its
-// Cholesky inverse, lambda and the fit; the I x R rows stay FP32.
+// Gauss-Jordan inverse, lambda and the fit; the I x R rows stay FP32.
 #pragma once
 
 #include "common.cuh"

@@ -23,6 +23,10 @@ namespace adatm {
 
 constexpr int kMaxModes = 8;  // device kernels support orders 3..8
 
+// SMs of a B200. Written out where work is split into chunks: the split, and
+// with it the last bits of the sums, does not depend on what a device reports.
+constexpr uint32_t kSms = 148;
+
 inline int ldr_of(uint64_t R) { return (int)((R + 3) / 4 * 4); }
 
 // (not volatile: a pure function of the lane, so the compiler may reuse it)

@@ -274,8 +274,8 @@ BatchSweep::BatchSweep(std::vector<Engine *> engines, cudaStream_t stream)
   if (e_.empty()) throw BadInput("an empty batch");
   for (Engine *e : e_)
     if (!e) throw BadInput("a null engine in the batch");
-  // the branches' walks run side by side: one chunk per warp, so their
-  // blocks interleave instead of each walk holding every SM in turn
+  // the branches' walks run side by side: one group of chunks per warp, so
+  // their blocks interleave instead of each walk holding every SM in turn
   for (Engine *e : e_) e->set_resident_grid(false);
   ADATM_CUDA(cudaEventCreateWithFlags(&fork_, cudaEventDisableTiming));
   join_.resize(e_.size(), nullptr);

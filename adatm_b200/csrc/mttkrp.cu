@@ -420,12 +420,6 @@ __host__ __device__ constexpr size_t scatter_warp_bytes(int ldr) {
           (size_t)kBatch * ldr * sizeof(float) + 15) / 16 * 16;
 }
 
-template <FactorType FT>
-__device__ __forceinline__ float4 ld_factor4(const void *U, uint32_t row, int ldr, int col, bool act) {
-  const fv<4> r = ld_factor<4, FT>(U, row, ldr, col, act);
-  return make_float4(r.x[0], r.x[1], r.x[2], r.x[3]);
-}
-
 // Prefix rows (per column, all ldr columns; rows ldr floats apart) of levels
 // lo..hi-1.
 template <FactorType FT>
@@ -529,7 +523,7 @@ __global__ void __launch_bounds__(256, HOT ? 3 : 1) k_scatter(const __grid_const
         constexpr int ST = 4;
         for (int k0 = k; k0 <= ke; k0 += ST * UPS) {
           float4 r[ST];
-          fv<4> m[LEAF ? 1 : ST];
+          float4 m[LEAF ? 1 : ST];
 #pragma unroll
           for (int t = 0; t < ST; ++t) {
             const int unit = k0 + t * UPS + slot;
@@ -537,7 +531,7 @@ __global__ void __launch_bounds__(256, HOT ? 3 : 1) k_scatter(const __grid_const
             r[t] = make_float4(1.f, 1.f, 1.f, 1.f);
             if (d >= 1) r[t] = ld_factor4<FT>(a.U[d - 1], pstage[__popc(M & ((1u << (unit & 31)) - 1u))],
                                               a.ldr, col, ok);
-            if constexpr (!LEAF) m[t] = ld_rows<4>(a.src_rows, base + (unit & 31), a.ldr, col, ok);
+            if constexpr (!LEAF) m[t] = ld_rows4(a.src_rows, base + (unit & 31), a.ldr, col, ok);
           }
 #pragma unroll
           for (int t = 0; t < ST; ++t) {
@@ -551,7 +545,7 @@ __global__ void __launch_bounds__(256, HOT ? 3 : 1) k_scatter(const __grid_const
               const float sv = __uint_as_float(e.y);
               x = make_float4(sv * p.x, sv * p.y, sv * p.z, sv * p.w);
             } else {
-              x = make_float4(m[t].x[0] * p.x, m[t].x[1] * p.y, m[t].x[2] * p.z, m[t].x[3] * p.w);
+              x = make_float4(m[t].x * p.x, m[t].y * p.y, m[t].z * p.z, m[t].w * p.w);
             }
             if (ok) {
               if (stage) sts4(xs + (unit & 31) * a.ldr + col, x);
@@ -751,10 +745,11 @@ void launch_contract_v(const WalkArgs &a, bool resident, cudaStream_t s) {
 // source units per node on average: at higher fan-out the extra row per unit
 // costs more than the closes it saves. `want` >= 0 caps the count.
 //
-// Measured (ms per MTTKRP, fold up to 4 / 10 / 30 units per node): FP32, R =
-// 32, the 6th-order tensor's second and third contractions 2.18 / 2.26 / 2.26
-// and 1.97 / 1.97 / 2.16; BF16 rows (half the L1 bytes per row), R = 64, the
-// 5th-order tensor's second contraction 1.44 / 1.25 / 1.25.
+// Measured (ms per MTTKRP, fold up to 4 / 10 / 30 units per node; the line lies
+// next to the best of them): FP32, R = 32, the 6th-order tensor's second and
+// third contractions 2.18 / 2.26 / 2.26 and 1.97 / 1.97 / 2.16; BF16 rows (half
+// the L1 bytes per row), R = 64, the 5th-order tensor's second contraction 1.44 /
+// 1.25 / 1.25.
 template <FactorType FT>
 constexpr double fold_units() {
   return FT == FactorType::F32 ? 5.0 : 10.0;
@@ -1027,7 +1022,7 @@ uint32_t auto_chunk(const TreeWalk &w) {
   if (w.src == w.out) return w.src == w.nmodes - 1 ? 2 * kScatterChunk : kScatterChunk;
   constexpr uint64_t kOnce = 128, kMinChunk = 16;
   const uint64_t most = w.R <= 32 ? 80 : 128, large = w.src == w.nmodes - 1 ? 256 : most;
-  const uint64_t slots = 148ull * 32 * default_walkers(w.R);
+  const uint64_t slots = kSms * 32ull * default_walkers(w.R);
   const uint64_t per_slot = (w.nunits + slots - 1) / slots;
   const uint64_t c = per_slot <= kOnce
                          ? per_slot

@@ -63,11 +63,11 @@ struct TreeWalk {
   DevBuf<uint32_t> sched;                    // nchunks x (S + 1), then the chunk counter
   bool resident = true;                      // contraction grid: resident blocks that claim
                                              // chunks (else a group of chunks per warp)
-  int walkers = 0;                           // contraction: walkers per warp (1, 2 or 4;
-                                             // 0 = default_walkers(R))
-  int fold = -1;                             // contraction: unstored levels above the
-                                             // source folded into its loop (0..2; -1 =
-                                             // as many as the tree's fan-out suggests)
+  int walkers = 0;                           // contraction: walkers per warp (1, 2 or 4; 0 =
+                                             // default_walkers(R), up to 8)
+  int fold = -1;                             // contraction: most unstored levels above the
+                                             // source folded into its loop (0..2; -1 = as
+                                             // many as the tree's fan-out suggests, up to 5)
   // Scatter walks: the output rows that the most units hit (at most
   // kHotRows, each hit by at least kHotMin units) are summed per block in
   // shared memory; hot_slot maps an output row to its slot (0xFF = none).

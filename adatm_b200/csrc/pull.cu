@@ -295,7 +295,7 @@ void pull_prepare(PullWalk &p, const DevCsf &c, int d, bool leaf, int R, int ldr
   // pulls, us with 16 / 32 / 64 / 128 / one per slot: R = 32, 97 units per slot 61 /
   // 62 / 61 / 65 / 61; 120 75 / 72 / 67 / 68 / 68; 130 78 / 76 / 75 / 84 / -; 208 115 / 112 /
   // 113 / 105 / -; 460 238 / 212 / 209 / 209 / -; R = 64, 132 per slot 76 / 70 / 73 / 84 / -
-  const uint64_t slots = 148ull * 32 * walkers_of(R), per_slot = (p.n + slots - 1) / slots;
+  const uint64_t slots = kSms * 32ull * walkers_of(R), per_slot = (p.n + slots - 1) / slots;
   const uint64_t u = per_slot <= 128 ? per_slot : std::min<uint64_t>(128, per_slot / 4);
   p.seg = (uint32_t)std::max<uint64_t>(16, (u + 15) / 16 * 16);
   p.nsegs = (uint32_t)((p.n + p.seg - 1) / p.seg);

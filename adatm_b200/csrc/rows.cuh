@@ -11,13 +11,6 @@ struct alignas(sizeof(float) * V) fv {
   float x[V];
 };
 
-template <int V>
-__device__ __forceinline__ fv<V> fv_fill(float s) {
-  fv<V> r;
-#pragma unroll
-  for (int i = 0; i < V; ++i) r.x[i] = s;
-  return r;
-}
 // Pairs of columns go through the packed FP32 instructions (one issue slot
 // for two products; each is rounded as its scalar form is).
 __device__ __forceinline__ uint64_t pack2(float x, float y) {
@@ -28,67 +21,25 @@ __device__ __forceinline__ uint64_t pack2(float x, float y) {
 __device__ __forceinline__ void unpack2(uint64_t p, float &x, float &y) {
   asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(p));
 }
-// Columns col..col+V-1 of factor row `row` (FP32 or BF16 storage).
-template <int V, FactorType FT>
-__device__ __forceinline__ fv<V> ld_factor(const void *U, uint32_t row, int ldr, int col, bool act) {
-  fv<V> r = fv_fill<V>(0.f);
-  if (!act) return r;
+// Columns col .. col+3 of factor row `row` (FP32 or BF16 storage).
+template <FactorType FT>
+__device__ __forceinline__ float4 ld_factor4(const void *U, uint32_t row, int ldr, int col, bool act) {
+  if (!act) return make_float4(0.f, 0.f, 0.f, 0.f);
   if constexpr (FT == FactorType::F32) {
-    const float *p = static_cast<const float *>(U) + (size_t)row * ldr + col;
-    if constexpr (V == 1) {
-      r.x[0] = __ldg(p);
-    } else if constexpr (V == 2) {
-      const float2 t = __ldg(reinterpret_cast<const float2 *>(p));
-      r.x[0] = t.x;
-      r.x[1] = t.y;
-    } else {
-      const float4 t = __ldg(reinterpret_cast<const float4 *>(p));
-      r.x[0] = t.x;
-      r.x[1] = t.y;
-      r.x[2] = t.z;
-      r.x[3] = t.w;
-    }
+    return __ldg(reinterpret_cast<const float4 *>(static_cast<const float *>(U) + (size_t)row * ldr + col));
   } else {
-    const __nv_bfloat16 *p = static_cast<const __nv_bfloat16 *>(U) + (size_t)row * ldr + col;
-    if constexpr (V == 1) {
-      r.x[0] = __bfloat162float(__ldg(p));
-    } else if constexpr (V == 2) {
-      const float2 t = __bfloat1622float2(__ldg(reinterpret_cast<const __nv_bfloat162 *>(p)));
-      r.x[0] = t.x;
-      r.x[1] = t.y;
-    } else {
-      const uint2 raw = __ldg(reinterpret_cast<const uint2 *>(p));
-      const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&raw.x));
-      const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&raw.y));
-      r.x[0] = lo.x;
-      r.x[1] = lo.y;
-      r.x[2] = hi.x;
-      r.x[3] = hi.y;
-    }
+    const uint2 raw = __ldg(
+        reinterpret_cast<const uint2 *>(static_cast<const __nv_bfloat16 *>(U) + (size_t)row * ldr + col));
+    const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&raw.x));
+    const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&raw.y));
+    return make_float4(lo.x, lo.y, hi.x, hi.y);
   }
-  return r;
 }
 
-// FP32 row matrices (memo rows, outputs).
-template <int V>
-__device__ __forceinline__ fv<V> ld_rows(const float *base, uint64_t row, int ldr, int col, bool act) {
-  fv<V> r = fv_fill<V>(0.f);
-  if (!act) return r;
-  const float *p = base + row * (uint64_t)ldr + col;
-  if constexpr (V == 1) {
-    r.x[0] = __ldg(p);
-  } else if constexpr (V == 2) {
-    const float2 t = __ldg(reinterpret_cast<const float2 *>(p));
-    r.x[0] = t.x;
-    r.x[1] = t.y;
-  } else {
-    const float4 t = __ldg(reinterpret_cast<const float4 *>(p));
-    r.x[0] = t.x;
-    r.x[1] = t.y;
-    r.x[2] = t.z;
-    r.x[3] = t.w;
-  }
-  return r;
+// And of an FP32 row matrix (memo rows).
+__device__ __forceinline__ float4 ld_rows4(const float *base, uint64_t row, int ldr, int col, bool act) {
+  if (!act) return make_float4(0.f, 0.f, 0.f, 0.f);
+  return __ldg(reinterpret_cast<const float4 *>(base + row * (uint64_t)ldr + col));
 }
 
 // FP64 output rows: the MTTKRP sums of a row can come from millions of
@@ -200,38 +151,6 @@ __device__ __forceinline__ Row<V> raw_row(const RawRow<V, FT> &a) {
         r.w[i] = pack2(__uint_as_float(a.w[i] << 16), __uint_as_float(a.w[i] & 0xFFFF0000u));
     }
     return r;
-  }
-}
-// Loaded where on != 0, without a branch; elsewhere the row keeps its value.
-template <int V, FactorType FT>
-__device__ __forceinline__ void ld_row_if(RawRow<V, FT> &a, const char *p, uint32_t on) {
-  if constexpr (FT == FactorType::F32) {
-    if constexpr (V == 1)
-      asm("{\n.reg .pred q;\nsetp.ne.u32 q, %2, 0;\n@q ld.global.nc.f32 %0, [%1];\n}"
-          : "+f"(a.r.w)
-          : "l"(p), "r"(on));
-    else if constexpr (V == 2)
-      asm("{\n.reg .pred q;\nsetp.ne.u32 q, %2, 0;\n@q ld.global.nc.b64 %0, [%1];\n}"
-          : "+l"(a.r.w[0])
-          : "l"(p), "r"(on));
-    else
-      asm("{\n.reg .pred q;\nsetp.ne.u32 q, %3, 0;\n@q ld.global.nc.v2.b64 {%0, %1}, [%2];\n}"
-          : "+l"(a.r.w[0]), "+l"(a.r.w[1])
-          : "l"(p), "r"(on));
-  } else {
-    if constexpr (V == 1)
-      asm("{\n.reg .pred q;\n.reg .b16 h;\nsetp.ne.u32 q, %2, 0;\n@q ld.global.nc.b16 h, [%1];\n"
-          "@q cvt.u32.u16 %0, h;\n}"
-          : "+r"(a.w[0])
-          : "l"(p), "r"(on));
-    else if constexpr (V == 2)
-      asm("{\n.reg .pred q;\nsetp.ne.u32 q, %2, 0;\n@q ld.global.nc.b32 %0, [%1];\n}"
-          : "+r"(a.w[0])
-          : "l"(p), "r"(on));
-    else
-      asm("{\n.reg .pred q;\nsetp.ne.u32 q, %3, 0;\n@q ld.global.nc.v2.b32 {%0, %1}, [%2];\n}"
-          : "+r"(a.w[0]), "+r"(a.w[1])
-          : "l"(p), "r"(on));
   }
 }
 template <int V, FactorType FT>

@@ -1,6 +1,7 @@
-// scan.cu -- exclusive prefix sums on the device, in three launches without
-// any inter-block waiting: per-tile sums, one block scanning the tile sums,
-// per-tile scans that add their tile offset.
+// scan.cu -- exclusive prefix sums on the device, without any inter-block
+// waiting: short arrays by one block, longer ones in three launches (per-tile
+// sums, one block scanning the tile sums, per-tile scans that add their tile
+// offset).
 #include "common.cuh"
 
 namespace adatm {

@@ -9,7 +9,7 @@ namespace {
 
 constexpr uint32_t kGroup = 64;  // partials that one walker (a group of lanes) adds
 constexpr uint32_t kMid = 64;    // groups under one group of groups, and most groups of a chain without
-constexpr uint32_t kWideGroups = 148 * 64;
+constexpr uint32_t kWideGroups = kSms * 64;
 // words of a chain: level, node, level slot, first boundary, partials, first
 // group, first group of groups, groups of groups (0 where the groups are few)
 constexpr int kChainWords = 8;
