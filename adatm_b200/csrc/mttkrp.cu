@@ -79,7 +79,7 @@ constexpr int kBatch = 32;  // units per batch of a scatter or pull warp
 // root walks against FP64, with one run and the value last / as here: the
 // 6th-order Zipf(1.3) tensor 3.4e-9, 4.6e-9, 8.7e-9 / 1.3e-9, 1.1e-9, 7.8e-10; the
 // 5th-order one, BF16 rows, 5.6e-9, 4.7e-9 / 1.8e-9, 2.2e-9. It costs these walks
-// 2.18, 2.04, 1.86 -> 2.23, 2.09, 1.90 ms and 2.26, 1.15 -> 2.33, 1.16 ms; with the
+// 2.18, 2.04, 1.86 -> 2.22, 2.08, 1.90 ms and 2.26, 1.15 -> 2.30, 1.16 ms; with the
 // sum held in registers, 2.26, 2.11, 1.91 and 2.41, 1.19.
 //
 // A node of level top that closes leaves the unit loop: its sum is stored
@@ -91,15 +91,16 @@ constexpr int kBatch = 32;  // units per batch of a scatter or pull warp
 // What bounds it: the L1 data pipe and the latency of the gathers behind it,
 // not DRAM. A row of R = 32 columns takes one of its cycles, so a unit takes
 // F + 1, next to about two for the staging and the closes. On the 6th-order
-// Zipf(1.3) tensor at 10.4M nonzeros (R = 32, F = 3) the pipe is busy 71% of
-// the time at 18 warp instructions per nonzero (issue 51%): 0.36 ms, against
+// Zipf(1.3) tensor at 10.4M nonzeros (R = 32, F = 3) the pipe is busy 68% of
+// the time at 19 warp instructions per nonzero (issue 50%): 0.38 ms, against
 // 0.47 ms and 29 instructions for one walk per warp whose closes went through
-// shared-memory items; the 77.9M-nonzero tensor's three contractions 2.32 /
-// 2.18 / 1.97 ms against 2.62 / 2.43 / 2.23. Measured and not kept: rows of
-// the folded levels kept across units and loaded under a predicate (a load
-// with inactive lanes costs the pipe as much as a full one), one unit in
-// flight with the next one's rows loaded ahead (2.33), three or five blocks
-// per SM (2.46 / 2.48), two walkers of two columns per lane (3.26).
+// shared-memory items; the 77.9M-nonzero tensor's three contractions 2.22 /
+// 2.08 / 1.90 ms against 2.62 / 2.43 / 2.23. Measured and not kept, when the first
+// of these took 2.31 ms: rows of the folded levels kept across units and loaded
+// under a predicate (a load with inactive lanes costs the pipe as much as a
+// full one), one unit in flight with the next one's rows loaded ahead (2.33),
+// three or five blocks per SM (2.46 / 2.48), two walkers of two columns per lane
+// (3.26).
 // ---------------------------------------------------------------------------
 constexpr int kMaxFold = 5;
 constexpr uint32_t kNoneHeld = 1u << 31;
@@ -163,12 +164,12 @@ __global__ void __launch_bounds__(256, 4)
       reinterpret_cast<uint32_t *>(reinterpret_cast<uint4 *>(wbase) + W * (B + 1)) + wk * (B + 1) * X;
   uint8_t *const scd =
       depth_bytes<W>() != 0 ? wbase + kStageBytes + wk * B : reinterpret_cast<uint8_t *>(stage + B);
+  // sum of the open level-top node in the batches before this one
+  Row<VW> *const held = reinterpret_cast<Row<VW> *>(wbase + kStageBytes + depth_bytes<W>()) + lane;
   // open node and open sum of level l in {d .. top-1}: nodes[l * 32], carry[l * 32]
-  uint32_t *const nodes = reinterpret_cast<uint32_t *>(wbase + kStageBytes + depth_bytes<W>()) + lane - d * 32;
+  uint32_t *const nodes = reinterpret_cast<uint32_t *>(held - lane + (W > 1 ? 32 : 0)) + lane - d * 32;
   Row<VW> *const carry =
       reinterpret_cast<Row<VW> *>(nodes + (top > d ? top : d) * 32 - lane) + lane - d * 32;
-  // sum of the open level-top node in the batches before this one
-  Row<VW> *const held = carry + (size_t)(top > d ? top : d) * 32;
   const int col = li * VW;
   const bool act = col < a.R;
   constexpr int esz = FT == FactorType::F32 ? 4 : 2;
@@ -180,7 +181,6 @@ __global__ void __launch_bounds__(256, 4)
   const uint32_t lane_off = (uint32_t)(act ? col : 0) * esz;
   const char *rows = static_cast<const char *>(hot.base) + lane_off;
   asm volatile("" : "+l"(rows));  // kept, not computed again at each load
-  const char *const rows_t = static_cast<const char *>(hot.top_rows) + lane_off;
   const uint32_t stride = (uint32_t)a.ldr * esz;
 
   // units whose rows are in flight together: as many as the registers hold
@@ -235,7 +235,7 @@ __global__ void __launch_bounds__(256, 4)
         return;
       }
       Row<VW> c = carry[(top - 1) * 32];
-      const Row<VW> row = ld_row<VW, FT>(row_at(rows_t, id, stride));
+      const Row<VW> row = ld_row<VW, FT>(row_at(static_cast<const char *>(hot.top_rows) + lane_off, id, stride));
       idt = __ldg(hot.top_ids + min(nt, hot.top_last));
       row_fma(c, x, row);
       int l = top - 1;
