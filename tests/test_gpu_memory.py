@@ -1,5 +1,7 @@
 """Device memory of the library: what it keeps for reuse is bounded and goes back
 when it is told to."""
+import gc
+
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -9,6 +11,7 @@ MIB = 1 << 20
 
 def free_bytes():
     import torch
+    gc.collect()  # engines of earlier tests that only a cycle holds
     torch.cuda.synchronize()
     return torch.cuda.mem_get_info()[0]
 
